@@ -877,7 +877,7 @@ struct TmapKeyHash {
   }
 };
 
-static int cached_tmap_2d_ld(CUtensorMap* out, const void* base, uint64_t rows, uint64_t k_elems, uint64_t ld, int elem_bytes,
+int cached_tmap_2d_ld(CUtensorMap* out, const void* base, uint64_t rows, uint64_t k_elems, uint64_t ld, int elem_bytes,
                              uint32_t box_rows) {
   static std::unordered_map<TmapKey, CUtensorMap, TmapKeyHash> cache;
   static std::mutex mu;

@@ -132,6 +132,7 @@ def lib():
     L = C.CDLL(str(_LIB_PATH), mode=C.RTLD_GLOBAL)
     vp, i32, i64, f32 = C.c_void_p, C.c_int, C.c_longlong, C.c_float
     _sig(L, "skein_gemm_ws", i32, [C.POINTER(GemmParams), vp])
+    _sig(L, "skein_gemm_pair", i32, [C.POINTER(GemmParams), vp])
     _sig(L, "skein_gemm_ws_workspace_bytes", i64, [C.POINTER(GemmParams)])
     _sig(L, "skein_sm_count", i32, [])
     _sig(L, "skein_reduce_residual_rmsnorm", i32,

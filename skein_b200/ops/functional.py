@@ -115,13 +115,31 @@ def pick_n_tile(rows_hint: int, dual: bool, features: int = 0) -> int:
     return max(16, min(cap, _round_up(max(rows_hint, 1), 16)))
 
 
-def _gemm_launch(p: "_lib.GemmParams", what: str, cfg: dict | None = None):
-    """Launch with (in this order) an explicit configuration, the measured one from the kernel-configuration cache
-    (tuning.py), or the heuristics below."""
+PAIR_MIN_ROWS = 96        # of a group
+
+
+def pair_gemm_ok(p: "_lib.GemmParams", rows: int) -> bool:
+    """Whether a product with `rows` rows in each of its groups runs on pairs of CTAs (csrc/kernels/gemm_pair.cu) instead of the streaming
+    kernel. Below that the weights' bytes decide and the streaming kernel, which spreads them over all SMs whatever the number of tiles, is
+    as quick or quicker; one group without a gate/up pair has few tiles, so that it changes sides later. Measured, streaming / pairs, us:
+    gate/up 14336 x 4096 53 / 56 at 64 rows, 60 / 58 at 96, 67 / 57 at 128, 150 / 89 at 512, 1080 / 608 at 4096; eight experts of it 296 / 285 at 64 rows
+    each, 312 / 294 at 96, 540 / 336 at 192; 10240 x 8192 57 / 61 at 128 rows, 67 / 65 at 192, 94 / 66 at 512, 673 / 444 at 4096."""
+    many = p.G > 1 or p.mode == 1
+    return rows >= (PAIR_MIN_ROWS if many else 2 * PAIR_MIN_ROWS) and p.F >= 256 and p.K >= 256
+
+
+def _gemm_launch(p: "_lib.GemmParams", what: str, cfg: dict | None = None, rows: int = 0):
+    """Launch with (in this order) an explicit configuration of the streaming kernel, the kernel for many rows (rows: of a group, as far as
+    the host knows; 0 keeps a product off it), the measured configuration from the kernel-configuration cache (tuning.py), or the
+    heuristics below."""
     ws = workspace()
     p.workspace = ws.gemm_ws.data_ptr()
     p.counters = ws.gemm_counters.data_ptr()
     p.status = ws.status.data_ptr()
+    if cfg is None and rows > 0 and pair_gemm_ok(p, rows):
+        _lib.check(_lib.lib().skein_gemm_pair(C.byref(p), _lib.stream_ptr()), what)
+        _lib.count_launch()
+        return
     p.line_cut_only = 1 if os.environ.get("SKEIN_GEMM_ALIGNED", "1") == "0" else 0
     if cfg is None:
         cache = tuning.active()
@@ -275,7 +293,7 @@ def linear(x, w, out=None, residual=None, n_tile=None, _cfg=None, out_f32=False,
         return out
     if tc_gemm_ok(x, K) and p.x_ld % 8 == 0 and x.data_ptr() % 16 == 0:
         _check_bf16(x)
-        _gemm_launch(p, "linear", _cfg)
+        _gemm_launch(p, "linear", _cfg, rows=0 if n_tile else T)
     else:
         simt_launch(p, x, T, "linear")
     return out
@@ -305,7 +323,7 @@ def swiglu_linear(x, w13, out=None, n_tile=None, _cfg=None, glu=None):
     if glu is not None:
         p.glu, p.glu_limit, p.glu_slope = 1, float(glu[0]), float(glu[1])
     if tc_gemm_ok(x, K):
-        _gemm_launch(p, "swiglu_linear", _cfg)
+        _gemm_launch(p, "swiglu_linear", _cfg, rows=0 if n_tile else T)
     else:
         simt_launch(p, x, T, "swiglu_linear")
     return out
@@ -337,8 +355,9 @@ def grouped_linear(xs, w, counts, offsets, swiglu=False, out=None, n_tile=None, 
             grouped_linear(xs, w[e0:e1], counts[e0:e1], offsets[e0:e1], swiglu, out, n_tile,
                            (rows_hint if rows_hint is not None else rows) * (e1 - e0) // E, grid, _cfg, glu)
         return out
+    avg = (rows_hint if rows_hint is not None else rows) / E
+    many = 0 if n_tile or grid else int(avg)
     if n_tile is None:
-        avg = (rows_hint if rows_hint is not None else rows) / E
         n_tile = pick_n_tile(int(math.ceil(avg * 1.5)), swiglu)
     wv, rows_pg, packed = _wview(w)
     p = _base_params(xs, wv, out, F, K, n_tile, 1 if swiglu else 0)
@@ -351,7 +370,7 @@ def grouped_linear(xs, w, counts, offsets, swiglu=False, out=None, n_tile=None, 
     if glu is not None:
         p.glu, p.glu_limit, p.glu_slope = 1, float(glu[0]), float(glu[1])
     if tc_gemm_ok(xs, K):
-        _gemm_launch(p, "grouped_linear", _cfg)
+        _gemm_launch(p, "grouped_linear", _cfg, rows=many)
     else:
         simt_launch(p, xs, rows, "grouped_linear")
     return out
