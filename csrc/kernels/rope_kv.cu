@@ -56,6 +56,52 @@ __global__ void rope_kv_append_kernel(__nv_bfloat16* __restrict__ qkv, const int
   dst[i + half] = __float2bfloat16(x1);
 }
 
+// The same with 16-byte accesses, D a multiple of 16 and 16-byte aligned rows: a CTA per token, a thread 8 rotation pairs of every
+// (threads / (D / 16))-th head, so that its cosines and sines are loaded once. What bounds it is the rows' bytes; with a thread per
+// pair and a CTA per head it was the number of 2-byte accesses and CTAs. 4096 tokens x 48 heads of 128: 103 -> 14 us.
+__global__ void __launch_bounds__(128) rope_kv_append_vec_kernel(__nv_bfloat16* __restrict__ qkv, const int* __restrict__ positions,
+                                                                 const int* __restrict__ seq_of_token, const int* __restrict__ block_table,
+                                                                 int max_blocks, const float* __restrict__ cos_sin,
+                                                                 __nv_bfloat16* __restrict__ kv_cache, int page_size, int Hq, int Hkv, int D,
+                                                                 int max_pos, int num_pages, int* status) {
+  const int t = blockIdx.x, half = D / 2, lanes = D / 16, heads_at_once = blockDim.x / lanes;
+  const int i = (threadIdx.x % lanes) * 8, head0 = threadIdx.x / lanes;
+  if (head0 >= heads_at_once) return;
+  const int pos = positions[t];
+  if (pos < 0) return;  // padding row of a captured batch bucket
+  if (pos >= max_pos) { report_status(status, ST_BAD_INDEX, pos); return; }
+  const int seq = seq_of_token ? seq_of_token[t] : t;
+  const int page = block_table[(size_t)seq * max_blocks + pos / page_size];
+  float c[8], sn[8];
+  const float4* cs = reinterpret_cast<const float4*>(cos_sin + ((size_t)pos * half + i) * 2);
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const float4 v = cs[k];
+    c[2 * k] = v.x; sn[2 * k] = v.y; c[2 * k + 1] = v.z; sn[2 * k + 1] = v.w;
+  }
+  for (int head = head0; head < Hq + 2 * Hkv; head += heads_at_once) {
+    __nv_bfloat16* row = qkv + ((size_t)t * (Hq + 2 * Hkv) + head) * D + i;
+    uint4 a = *reinterpret_cast<const uint4*>(row), b = *reinterpret_cast<const uint4*>(row + half);
+    if (head < Hq + Hkv) {
+      __nv_bfloat162 *ab = reinterpret_cast<__nv_bfloat162*>(&a), *bb = reinterpret_cast<__nv_bfloat162*>(&b);
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const float2 x0 = __bfloat1622float2(ab[k]), x1 = __bfloat1622float2(bb[k]);
+        ab[k] = __floats2bfloat162_rn(x0.x * c[2 * k] - x1.x * sn[2 * k], x0.y * c[2 * k + 1] - x1.y * sn[2 * k + 1]);
+        bb[k] = __floats2bfloat162_rn(x1.x * c[2 * k] + x0.x * sn[2 * k], x1.y * c[2 * k + 1] + x0.y * sn[2 * k + 1]);
+      }
+    }
+    __nv_bfloat16* dst = row;
+    if (head >= Hq) {
+      const int is_v = head >= Hq + Hkv, kvh = head - Hq - (is_v ? Hkv : 0);
+      if (page < 0 || page >= num_pages) { report_status(status, ST_BAD_INDEX, page); return; }
+      dst = kv_cache + ((((size_t)page * 2 + is_v) * Hkv + kvh) * page_size + pos % page_size) * D + i;
+    }
+    *reinterpret_cast<uint4*>(dst) = a;
+    *reinterpret_cast<uint4*>(dst + half) = b;
+  }
+}
+
 // out[t, :] = table[ids[t] - vocab_start, :] if the id falls in this rank's vocabulary shard, else 0.
 __global__ void embed_gather_kernel(const int* __restrict__ ids, const __nv_bfloat16* __restrict__ table,
                                     __nv_bfloat16* __restrict__ out, int H, int vocab_start, int vocab_rows) {
@@ -98,6 +144,12 @@ extern "C" int skein_rope_kv_append(void* qkv, const int* positions, const int* 
                                     int Hkv, int D, int max_pos, int num_pages, int* status, void* stream) {
   if (T == 0) return 0;
   if (D % 2 != 0 || D / 2 > 1024) return -1;
+  if (D % 16 == 0 && D <= 2048 && (((uintptr_t)qkv | (uintptr_t)kv_cache | (uintptr_t)cos_sin) & 15) == 0) {
+    skein::rope_kv_append_vec_kernel<<<T, 128, 0, (cudaStream_t)stream>>>(
+        (__nv_bfloat16*)qkv, positions, seq_of_token, block_table, max_blocks, cos_sin, (__nv_bfloat16*)kv_cache,
+        page_size, Hq, Hkv, D, max_pos, num_pages, status);
+    return (int)cudaGetLastError();
+  }
   dim3 grid(T, Hq + 2 * Hkv);
   skein::rope_kv_append_kernel<<<grid, D / 2, 0, (cudaStream_t)stream>>>(
       (__nv_bfloat16*)qkv, positions, seq_of_token, block_table, max_blocks, cos_sin, (__nv_bfloat16*)kv_cache,
