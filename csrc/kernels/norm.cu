@@ -210,6 +210,83 @@ __global__ void __launch_bounds__(512) reduce_residual_rmsnorm_kernel(const Norm
   reduce_norm_row<MAX_PASSES>(p, blockIdx.x, sh, wait_failed, nb);
 }
 
+// Many rows of one local source (prefill chunks), TK slots per row. What bounds it is the rows' bytes; the kernel above keeps one CTA of 512
+// threads per SM (its loads of up to 8 sources and 8 slots take the registers), each with one 16-byte load per thread in flight. Here a row
+// takes H / 32 threads with four loads of every operand in flight, and an SM holds several rows.
+// 4096 rows x 4096: 74 -> 21 us from one partial (6.4 TB/s), 102 -> 32 from two slots, 44 -> 17 without one.
+constexpr int ROWS_VEC = 4;
+template <int TK>
+__global__ void __launch_bounds__(512) reduce_norm_rows_kernel(const NormParams p) {
+  __shared__ float sh[32];
+  pdl_trigger();
+  pdl_wait();
+  const int b = blockIdx.x, step = blockDim.x * 8;
+  int row[TK];
+  float w[TK];
+#pragma unroll
+  for (int j = 0; j < TK; ++j) {
+    row[j] = p.row_idx ? p.row_idx[b * TK + j] : b;
+    w[j] = p.row_w ? p.row_w[b * TK + j] : 1.f;
+  }
+  uint4 r[ROWS_VEC], q[TK][ROWS_VEC];
+#pragma unroll
+  for (int v = 0; v < ROWS_VEC; ++v) {
+    const int h = threadIdx.x * 8 + v * step;
+    r[v] = make_uint4(0, 0, 0, 0);
+    if (h < p.H && p.residual) r[v] = *reinterpret_cast<const uint4*>(p.residual + (size_t)b * p.H + h);
+#pragma unroll
+    for (int j = 0; j < TK; ++j) {
+      q[j][v] = make_uint4(0, 0, 0, 0);
+      if (h < p.H && p.partial && row[j] >= 0) q[j][v] = __ldcg(reinterpret_cast<const uint4*>(p.partial + (size_t)row[j] * p.H + h));
+    }
+  }
+  float ss = 0.f;
+#pragma unroll
+  for (int v = 0; v < ROWS_VEC; ++v) {
+    const int h = threadIdx.x * 8 + v * step;
+    __nv_bfloat162* rb = reinterpret_cast<__nv_bfloat162*>(&r[v]);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      float2 a = __bfloat1622float2(rb[i]);
+      if (p.partial) {
+#pragma unroll
+        for (int j = 0; j < TK; ++j) {
+          if (row[j] < 0) continue;  // pair routed to an expert that lives on another rank
+          const float2 f = __bfloat1622float2(reinterpret_cast<const __nv_bfloat162*>(&q[j][v])[i]);
+          a.x += w[j] * f.x; a.y += w[j] * f.y;
+        }
+      }
+      rb[i] = __floats2bfloat162_rn(a.x, a.y);
+      const float2 f = __bfloat1622float2(rb[i]);       // the residual stream is bf16: the rounded value is normalised
+      ss += f.x * f.x + f.y * f.y;
+    }
+    if (h < p.H && p.residual_out) *reinterpret_cast<uint4*>(p.residual_out + (size_t)b * p.H + h) = r[v];
+  }
+  if (p.gamma == nullptr || p.normed_out == nullptr) return;
+  uint4 g[ROWS_VEC];
+#pragma unroll
+  for (int v = 0; v < ROWS_VEC; ++v) {
+    const int h = threadIdx.x * 8 + v * step;
+    if (h < p.H) g[v] = *reinterpret_cast<const uint4*>(p.gamma + h);
+  }
+  const float inv = rsqrtf(block_sum(ss, sh) / (float)p.H + p.eps);
+#pragma unroll
+  for (int v = 0; v < ROWS_VEC; ++v) {
+    const int h = threadIdx.x * 8 + v * step;
+    if (h >= p.H) break;
+    uint4 o;
+    const __nv_bfloat162 *rb = reinterpret_cast<const __nv_bfloat162*>(&r[v]), *gb = reinterpret_cast<const __nv_bfloat162*>(&g[v]);
+    __nv_bfloat162* ob = reinterpret_cast<__nv_bfloat162*>(&o);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const float2 f = __bfloat1622float2(rb[i]), gf = __bfloat1622float2(gb[i]);
+      const float2 xf = __bfloat1622float2(__floats2bfloat162_rn(f.x * inv, f.y * inv));      // rounded like the kernel above
+      ob[i] = __floats2bfloat162_rn(xf.x * gf.x, xf.y * gf.y);
+    }
+    *reinterpret_cast<uint4*>(p.normed_out + (size_t)b * p.H + h) = o;
+  }
+}
+
 // ---------------------------------------------------------------------------------------------
 // The same row reduction followed, in the same launch, by the MoE router and the scatter of the
 // normalised row into expert-sorted order (decode steps: every token's CTA is resident at once).
@@ -288,10 +365,15 @@ extern "C" int skein_reduce_residual_rmsnorm(
   p.flags = flags; p.epoch = epoch; p.status = status; p.src_stride = src_stride;
   p.B = B; p.H = H; p.n_src = n_src; p.topk = topk; p.eps = eps;
   p.budget_ns = (unsigned long long)(wait_budget_ms > 0 ? wait_budget_ms : 10000) * 1000000ull;
+  cudaStream_t s = (cudaStream_t)stream;
+  // two rows per SM and more: rows in flight count, not the latency of one (296 rows x 4096: 5.5 -> 3.2 us)
+  if (B >= 2 * 148 && !p.use_ptrs && flags == nullptr && owner_ids == nullptr && (partial == nullptr || n_src == 1) && topk <= 2) {
+    const dim3 block(((H + 8 * ROWS_VEC - 1) / (8 * ROWS_VEC) + 31) & ~31);
+    return (int)(topk == 2 ? launch_pdl(reduce_norm_rows_kernel<2>, dim3(B), block, 0, s, p) : launch_pdl(reduce_norm_rows_kernel<1>, dim3(B), block, 0, s, p));
+  }
   int threads = (H / 8 + 31) / 32 * 32;
   if (threads > 512) threads = 512;
   const int passes = (H + threads * 8 - 1) / (threads * 8);
-  cudaStream_t s = (cudaStream_t)stream;
   if (passes <= 1) return (int)launch_pdl(reduce_residual_rmsnorm_kernel<1>, dim3(B), dim3(threads), 0, s, p);
   if (passes <= 2) return (int)launch_pdl(reduce_residual_rmsnorm_kernel<2>, dim3(B), dim3(threads), 0, s, p);
   return (int)launch_pdl(reduce_residual_rmsnorm_kernel<4>, dim3(B), dim3(threads), 0, s, p);
