@@ -1,8 +1,8 @@
 """Prefill attention, two heads of a group per CTA (csrc/kernels/attn_prefill_tc.cu), against the operator's fp32 reference at the edges of its tiles.
 
-Bound per output: the probabilities are rounded to bf16, 2^-9 of each, in the weighted sum of the values and in the sum that divides it, which
-moves the result by at most 2 * 2^-9 of the weighted sum of the values' magnitudes; the result is rounded to bf16, 2^-9 of it. A tenth more covers the fp32 scores
-and exponentials.
+Bound per output: the probabilities are rounded to bf16, at most 2^-8 of each, in the weighted sum of the values and in the sum that divides it,
+which moves the result by at most 2 * 2^-8 of the weighted sum of the values' magnitudes; the result is rounded to bf16, 2^-8 of it. A tenth more covers
+the fp32 scores and exponentials.
 """
 import pytest
 import torch
@@ -41,5 +41,5 @@ def test_tiles(new, cached, heads, kv_heads):
     size[:, 1] = clean[:, 1].abs()
     cpu = [t.cpu() for t in args]
     want, mass = (ref.attn_prefill(q.float().cpu(), c.float(), table.cpu(), *cpu, heads, kv_heads, D) for c in (clean, size))
-    bound = 1.1 * (2.0 ** -8 * mass.float() + 2.0 ** -8 * want.float().abs())
+    bound = 1.1 * (2 * 2.0 ** -8 * mass.float() + 2.0 ** -8 * want.float().abs())
     assert bool(((y.float().cpu() - want.float()).abs() <= bound).all())
