@@ -126,6 +126,14 @@ __device__ __forceinline__ void build_sched(Sched& sched, const SkeinGemmParams&
     if (sp > 8) sp = 8;
     const int by_k = sched.KB / 4 > 0 ? sched.KB / 4 : 1;   // at least 4 K-blocks per piece
     if (sp > by_k) sp = by_k;
+    if (k_elems_per_block == 128) {
+      // e4m3 weights: a K-block costs a CTA its conversion whatever the memory does, so the longest piece decides and an idle CTA is lost.
+      // Aligned pieces while they are at most 6 K-blocks longer than an equal share, which is what its second partial tile costs:
+      // 10240 x 8192 (80 tiles of 64, whole) 38.9 against 32.8 us, 8192 x 28672 (64 of 224 in two) 67.6 / 62.8, 8192 x 8192 27.1 / 27.7,
+      // gate/up 3584 x 8192 (28 of 64 in five) 23.6 / 27.1
+      if ((sched.KB + sp - 1) / sp <= (int)((sched.TK + grid - 1) / grid) + 6) sched.split = sp;
+      return;
+    }
     // with fewer than two CTAs per tile, whole tiles on `acc` CTAs beat the line cut while the longer
     // K loop costs less than the second partial tile that the line cut's straddling brings
     if (sp >= 2 || (long long)sched.KB * (grid - acc) < 30ll * grid) sched.split = sp;

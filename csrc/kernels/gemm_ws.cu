@@ -49,11 +49,11 @@ constexpr int BLOCK_KB = 128;     // bytes of K per stage row (64 bf16 or 128 e4
 constexpr int W_TILE_BYTES = TILE_F * BLOCK_KB;  // 16 KB
 constexpr int ACC_STRIDE_MAX = 256;   // TMEM columns per accumulator buffer, at most
 constexpr int NUM_THREADS = 192;
-constexpr int W8_CONV_THREADS = 256;
-constexpr int W8_THREADS = NUM_THREADS + W8_CONV_THREADS;   // + 8 converter warps (e4m3 -> scaled bf16 in shared memory)
+constexpr int W8_GROUPS = 2;      // groups of four converter warps (e4m3 -> scaled bf16 in tensor memory; at most as many as slots: see plan())
+constexpr int W8_THREADS = NUM_THREADS + W8_GROUPS * 128;
 constexpr int EPI_THREADS = 128;
 constexpr int MAX_STAGES = 12;
-constexpr int W8_CONV_SLOTS = 3;  // ring of converted half K-blocks in tensor memory (64 K elements = 32 columns per weight tile)
+constexpr int W8_CONV_SLOTS = 6;  // ring of converted K-blocks in tensor memory, as many as fit (128 K elements = 64 columns per weight tile)
 constexpr int W8_SLOT_COLS = 32;  // 32-bit columns of one converted weight tile half: 64 bf16 K elements, two per column
 
 // Optional phase timer (compile with -DSKEIN_GEMM_TIMING): every CTA records %globaltimer at the points marked
@@ -74,6 +74,14 @@ __device__ unsigned long long g_w8_prof[160][8];
 #define PROF_T0() do { } while (0)
 #define PROF_ADD(i) do { } while (0)
 #endif
+
+// Position in a ring of barriers (a remainder by a number that is known at run time costs a role that walks one 16 KB tile per 0.4 us its pace).
+struct Ring {
+  uint32_t i = 0, phase = 0;
+  __device__ __forceinline__ void step(uint32_t n) {
+    if (++i == n) { i = 0; phase ^= 1; }
+  }
+};
 
 struct KernelArgs {
   SkeinGemmParams p;
@@ -147,7 +155,7 @@ gemm_ws_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ 
     }
     if (W8) {
       for (int c = 0; c < a.conv_slots; ++c) {
-        mbar_init(smem_u32(&bar_cfull[c]), W8_CONV_THREADS);
+        mbar_init(smem_u32(&bar_cfull[c]), 128);
         mbar_init(smem_u32(&bar_cempty[c]), 1);
       }
     }
@@ -191,7 +199,7 @@ gemm_ws_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ 
         uint32_t tx_bytes = (DUAL ? 2 : 1) * W_TILE_BYTES + a.x_tile_bytes;
         const uint32_t tx_base = tx_bytes;
         const long long w_rows_total = (long long)p.G * p.w_rows_per_group;
-        uint32_t it = 0;
+        Ring stage;
         int pos = kb_begin;
         bool ok = true;
         while (pos < kb_end && ok) {
@@ -208,9 +216,8 @@ gemm_ws_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ 
           const bool scales_by_copy = W8 && (w_row + (DUAL ? p.up_row_off : 0) + TILE_F <= w_rows_total) &&
                                       (un.m * TILE_F + TILE_F <= p.F) && (w_rows_total % 4 == 0) && (p.up_row_off % 4 == 0);
           if (W8) tx_bytes = tx_base + (scales_by_copy ? (DUAL ? 2 : 1) * 512u : 0u);
-          for (int kb = kb0; kb < kb1; ++kb, ++it) {
-            const uint32_t s = it % a.stages;
-            const uint32_t ph = (it / a.stages) & 1;
+          for (int kb = kb0; kb < kb1; ++kb, stage.step(a.stages)) {
+            const uint32_t s = stage.i, ph = stage.phase;
             {
               PROF_T0();
               if (!mbar_wait(smem_u32(&bar_empty[s]), ph ^ 1, &abort_flag, a.budget_ns)) {
@@ -250,7 +257,7 @@ gemm_ws_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ 
       // ================= MMA issuer =================
       if (elect_one()) {
         const uint32_t idesc = umma_idesc(1, 1, TILE_F, n_tile);
-        uint32_t it = 0;
+        Ring stage, slot;
         uint32_t seg = 0;
         int pos = kb_begin;
         bool ok = true;
@@ -268,13 +275,13 @@ gemm_ws_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ 
           }
           tc_fence_after();
           const uint32_t d_tmem = tmem_base + b * a.acc_stride;
-          for (int kb = kb0; kb < kb1; ++kb, ++it) {
-            const uint32_t s = it % a.stages;
-            const uint32_t ph = (it / a.stages) & 1;
+          for (int kb = kb0; kb < kb1; ++kb, stage.step(a.stages)) {
+            const uint32_t s = stage.i, ph = stage.phase;
             const uint32_t st = smem_base + s * a.stage_bytes;
             if (W8) {
               // the converted weights of this stage arrive from the converter warps in one slot of the tensor-memory ring
-              const uint32_t c = it % a.conv_slots, cph = (it / a.conv_slots) & 1;
+              const uint32_t c = slot.i, cph = slot.phase;
+              slot.step(a.conv_slots);
               {
                 PROF_T0();
                 if (!mbar_wait(smem_u32(&bar_cfull[c]), cph, &abort_flag, a.budget_ns)) {
@@ -287,7 +294,7 @@ gemm_ws_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ 
               }
               PROF_T0();
               tc_fence_after();
-              if (it == 0) TS(2);
+              if (seg == 0 && kb == kb0) TS(2);
               const uint32_t aw = tmem_base + a.conv_base + c * W8_SLOT;
 #pragma unroll
               for (int h = 0; h < 2; ++h) {          // K halves of the stage: 64 K elements = 4 MMAs of 16 (8 columns of A each)
@@ -316,7 +323,7 @@ gemm_ws_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ 
               break;
             }
             tc_fence_after();
-            if (it == 0) TS(2);
+            if (seg == 0 && kb == kb0) TS(2);
             const uint64_t dw = umma_desc_sw128(st);
             const uint64_t dx = umma_desc_sw128(st + W_STAGE_BYTES);
 #pragma unroll
@@ -338,20 +345,20 @@ gemm_ws_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ 
       }
     } else if (W8 && warp >= 6) {
       // ================= converters (warps 6..13): e4m3 tile -> bf16 rows, scaled by the row's 1 x 128 block scale, in TMEM ==
-      // Two threads share weight row r of the tile, each taking two of the four 16-byte chunks of a 64-K half (eight
-      // warps: two per scheduler, so that one warp's dependent instructions are covered by the other's). The raw tile
-      // was written by TMA with the 128-byte swizzle (16-byte chunk c of row r sits at chunk c ^ (r & 7)). A warp can
-      // reach the tensor-memory lanes 32 * (warp % 4) .. + 31 only, and lane = row of the A operand, so a warp converts
-      // the rows of its own lane quarter; 16 K elements become 8 columns.
+      // Two groups of four warps take the stages in turn, so that one group's chain (wait for the tile, for the slot, load, convert, store,
+      // wait for the stores, hand over) is covered by the other's: with all warps on one stage that chain was 0.45 of the 0.7 us that a
+      // 16 KB stage took. With as many slots as fit instead of three: 8192 x 28672 at 32 tokens 82 -> 66 -> 56 us, eight experts of 4096 x 14336 at 8 rows
+      // 136 -> 107 -> 96 (4.9 TB/s), their gate/up 186 -> 163 -> 162 (6.0 TB/s). Three groups leave 96 registers per thread and are slower. A thread converts one
+      // weight row. The raw tile was written by TMA with the 128-byte swizzle (16-byte chunk c of row r sits at chunk
+      // c ^ (r & 7)). A warp can reach the tensor-memory lanes 32 * (warp % 4) .. + 31 only, and lane = row of the A operand, so a warp
+      // converts the rows of its own lane quarter; 16 K elements become 8 columns.
       const int r = (warp & 3) * 32 + lane;
-      const int part = (warp - 6) >> 2;                      // which two chunks of every half this thread converts
+      const uint32_t group = (warp - 6) >> 2;
       const long long w_rows_total = (long long)p.G * p.w_rows_per_group;
-      uint32_t it = 0;
+      Ring stage, slot;
+      uint32_t turn = 0;
       int pos = kb_begin;
       bool ok = true;
-      // The hand-over of a converted half to the MMA warp is deferred by one step: its tensor-memory stores complete
-      // while the next half is loaded and converted, so the wait for them costs nothing when it finally comes.
-      int pending_slot = -1;
       while (pos < kb_end && ok) {
         const int u = pos / KB;
         const int kb0 = pos - u * KB;
@@ -361,8 +368,9 @@ gemm_ws_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ 
         const long long w_row = (long long)un.g * p.w_rows_per_group + un.m * TILE_F + r;
         const bool scales_by_copy = ((long long)un.g * p.w_rows_per_group + un.m * TILE_F + (DUAL ? p.up_row_off : 0) + TILE_F <= w_rows_total) &&
                                     (un.m * TILE_F + TILE_F <= p.F) && (w_rows_total % 4 == 0) && (p.up_row_off % 4 == 0);
-        for (int kb = kb0; kb < kb1 && ok; ++kb, ++it) {
-          const uint32_t s = it % a.stages, ph = (it / a.stages) & 1;
+        for (int kb = kb0; kb < kb1 && ok; ++kb, stage.step(a.stages), slot.step(a.conv_slots), turn ^= 1) {
+          if (turn != group) continue;
+          const uint32_t s = stage.i, ph = stage.phase, c = slot.i, cph = slot.phase;
           {
             PROF_T0();
             if (!mbar_wait(smem_u32(&bar_full[s]), ph, &abort_flag, a.budget_ns)) {
@@ -371,7 +379,7 @@ gemm_ws_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ 
               ok = false;
               break;
             }
-            if (r == 0 && part == 0) PROF_ADD(0);
+            if (r == 0) PROF_ADD(0);
           }
           // shared-memory addresses (32-bit, shared state space): loads and stores below are ld.shared / st.shared, not
           // generic accesses, which the hardware tracks like global ones (they showed up as the kernel's dominant stall)
@@ -388,7 +396,6 @@ gemm_ws_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ 
             const __nv_bfloat162 hs = __float2bfloat162_rn(f * 0x1p120f);
             sc[t] = *reinterpret_cast<const uint32_t*>(&hs);
           }
-          const uint32_t c = it % a.conv_slots, cph = (it / a.conv_slots) & 1;
           {
             PROF_T0();
             if (!mbar_wait(smem_u32(&bar_cempty[c]), cph ^ 1, &abort_flag, a.budget_ns)) {
@@ -397,60 +404,42 @@ gemm_ws_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ 
               ok = false;
               break;
             }
-            if (r == 0 && part == 0) PROF_ADD(1);
+            if (r == 0) PROF_ADD(1);
           }
           PROF_T0();
           tc_fence_after();
+          const uint32_t conv = tmem_base + ((uint32_t)((warp & 3) * 32) << 16) + a.conv_base + c * W8_SLOT;
 #pragma unroll
-          for (int h = 0; h < W8_PAIRS; ++h) {
-            // this thread's 16 columns of its lane in each of the pair's two sub-tiles: slot c, pair h, sub-tile t, columns
-            // part * 16 .. + 15. Sub-tile t is tile t (gate / up) at K half h with a pair of tiles, else K half t of the one tile.
-            const uint32_t conv = tmem_base + ((uint32_t)((warp & 3) * 32) << 16) + a.conv_base + c * W8_SLOT +
-                                  h * 2 * W8_SLOT_COLS + part * 16;
-            uint32_t o[2][16];
-            uint4 v[2][2];
+          for (int t = 0; t < (DUAL ? 2 : 1); ++t) {
+            const uint32_t src_row = raw + t * W_TILE_BYTES + r * 128;
 #pragma unroll
-            for (int t = 0; t < 2; ++t) {
-              const uint32_t src_row = raw + (DUAL ? t : 0) * W_TILE_BYTES + r * 128;
-              const int half = DUAL ? h : t;
+            for (int h = 0; h < 2; ++h) {      // K halves of 64: with a gate/up pair the two tiles' columns alternate
+              uint4 v[4];
 #pragma unroll
-              for (int ci = 0; ci < 2; ++ci)             // this thread's 16-byte chunks of e4m3, all loads first
-                asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];"
-                             : "=r"(v[t][ci].x), "=r"(v[t][ci].y), "=r"(v[t][ci].z), "=r"(v[t][ci].w)
-                             : "r"(src_row + (((half * 4 + part * 2 + ci) ^ (r & 7)) << 4)));
-            }
+              for (int ci = 0; ci < 4; ++ci)
+                asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v[ci].x), "=r"(v[ci].y), "=r"(v[ci].z), "=r"(v[ci].w)
+                             : "r"(src_row + (((h * 4 + ci) ^ (r & 7)) << 4)));
+              uint32_t o[32];
 #pragma unroll
-            for (int t = 0; t < 2; ++t) {
-              const uint32_t sct = sc[DUAL ? t : 0];
-#pragma unroll
-              for (int ci = 0; ci < 2; ++ci) {
-                e4m3x4_to_scaled_bf16x4(v[t][ci].x, sct, o[t][8 * ci + 0], o[t][8 * ci + 1]);
-                e4m3x4_to_scaled_bf16x4(v[t][ci].y, sct, o[t][8 * ci + 2], o[t][8 * ci + 3]);
-                e4m3x4_to_scaled_bf16x4(v[t][ci].z, sct, o[t][8 * ci + 4], o[t][8 * ci + 5]);
-                e4m3x4_to_scaled_bf16x4(v[t][ci].w, sct, o[t][8 * ci + 6], o[t][8 * ci + 7]);
+              for (int ci = 0; ci < 4; ++ci) {
+                e4m3x4_to_scaled_bf16x4(v[ci].x, sc[t], o[8 * ci + 0], o[8 * ci + 1]);
+                e4m3x4_to_scaled_bf16x4(v[ci].y, sc[t], o[8 * ci + 2], o[8 * ci + 3]);
+                e4m3x4_to_scaled_bf16x4(v[ci].z, sc[t], o[8 * ci + 4], o[8 * ci + 5]);
+                e4m3x4_to_scaled_bf16x4(v[ci].w, sc[t], o[8 * ci + 6], o[8 * ci + 7]);
               }
+              const uint32_t at = conv + (DUAL ? h * 2 + t : h) * W8_SLOT_COLS;
+              tmem_st16(at, o);
+              tmem_st16(at + 16, o + 16);
             }
-            if (h == 0 && pending_slot >= 0) {
-              // the previous stage's stores to tensor memory have had this conversion to complete
-              tmem_st_wait();
-              tc_fence_before();
-              mbar_arrive(smem_u32(&bar_cfull[pending_slot]));
-            }
-#pragma unroll
-            for (int t = 0; t < 2; ++t) tmem_st16(conv + t * W8_SLOT_COLS, o[t]);
           }
-          pending_slot = (int)c;
+          tmem_st_wait();
+          tc_fence_before();
+          mbar_arrive(smem_u32(&bar_cfull[c]));
 #ifdef SKEIN_GEMM_TIMING
-          if (r == 0 && part == 0) { PROF_ADD(2); g_w8_prof[blockIdx.x][6] += 1; }
+          if (r == 0) { PROF_ADD(2); g_w8_prof[blockIdx.x][6] += 1; }
 #endif
         }
         pos = u * KB + kb1;
-      }
-      if (pending_slot >= 0) {
-        // (also on the way out after a failed wait: the MMA warp gives up on the abort flag, an extra arrival is harmless)
-        tmem_st_wait();
-        tc_fence_before();
-        mbar_arrive(smem_u32(&bar_cfull[pending_slot]));
       }
     } else if (warp < 6) {
       // ================= epilogue (warps 2..5) =================
@@ -977,6 +966,10 @@ static int plan(const SkeinGemmParams* p, KernelArgs* ka, int* grid, size_t* sme
   int st = budget / ka->stage_bytes;
   if (st > MAX_STAGES) st = MAX_STAGES;
   if (p->stages > 0 && p->stages < st) st = p->stages;
+  // A converter group sees every second stage only, and its wait for a barrier's phase is good only while the phase before is known to be
+  // over: its own stage before says so for a slot (the MMAs of two stages and one turn of the slots earlier are done, and there are at least two
+  // slots), and for a stage if the same group had the stage that was in this place before, or if that one is as long gone.
+  if (w8 && st % W8_GROUPS != 0 && st < W8_GROUPS + ka->conv_slots) --st;
   if (st < 2) return -7;
   ka->stages = st;
   ka->budget_ns = (uint64_t)(p->wait_budget_ms > 0 ? p->wait_budget_ms : gemm_wait_budget_ms()) * 1000000ull;
