@@ -22,8 +22,10 @@ and are skipped by the kernels.
 """
 from __future__ import annotations
 
+import itertools
 import os
 
+import numpy as np
 import torch
 
 from .. import ops
@@ -336,22 +338,44 @@ class ModelRunner:
     def _prefill_inputs(self, seqs, sampling, want=None):
         """BatchInputs (and SamplingInputs) of one eager chunk holding every new token of every listed sequence. `want` lists, per
         sequence, the places among its new tokens that produce logits (default: the last one)."""
-        dev = self.device
-        toks, pos, sot, qs, ql, kl, rows, slots = [], [], [], [], [], [], [], []
-        S = len(seqs)
-        bt = torch.zeros(S, self.max_blocks, dtype=torch.int32)
-        for s, (ids, table, cached, *slot) in enumerate(seqs):
-            slots.append(slot[0] if slot else s)
-            qs.append(len(toks)); ql.append(len(ids)); kl.append(cached + len(ids))
-            toks.extend(ids); pos.extend(range(cached, cached + len(ids))); sot.extend([s] * len(ids))
-            rows.extend([len(toks) - 1] if want is None else [qs[-1] + i for i in want[s]])
-            bt[s, :len(table)] = torch.as_tensor(table, dtype=torch.int32)
-        i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=dev)
-        inp = BatchInputs(token_ids=i32(toks), positions=i32(pos), block_table=bt.to(dev), seq_lens=i32(kl),
-                          is_prefill=True, seq_of_token=i32(sot), q_start=i32(qs), q_len=i32(ql), max_q_len=max(ql),
-                          logit_rows=torch.tensor(rows, dtype=torch.int64, device=dev), kv_start=i32([sum(kl[:i]) for i in range(S)]),
-                          kv_total=sum(kl), max_cached=max(k - q for k, q in zip(kl, ql)),
-                          slots=i32(slots) if self.stateful else None)
+        dev, S = self.device, len(seqs)
+        plain = lambda v: v.tolist() if torch.is_tensor(v) else v      # noqa: E731
+        ql = [len(s[0]) for s in seqs]
+        kl = [s[2] + n for s, n in zip(seqs, ql)]
+        qs, ks = [0], [0]
+        for n, k in zip(ql, kl):
+            qs.append(qs[-1] + n)
+            ks.append(ks[-1] + k)
+        rows = [e - 1 for e in qs[1:]] if want is None else [qs[s] + i for s in range(S) for i in want[s]]
+        # One pinned buffer and one copy to the device. A tensor from a list for each of the ten inputs, copied from pageable memory, kept
+        # the device waiting 0.2 ms for a short prompt and 0.8 ms for a chunk of 4096 tokens.
+        sizes = {"rows": 2 * len(rows), "tok": qs[-1], "pos": qs[-1], "sot": qs[-1], "qs": S, "ql": S, "kl": S, "ks": S, "slots": S,
+                 "bt": S * self.max_blocks}
+        at, total = {}, 0
+        for name, n in sizes.items():
+            at[name] = slice(total, total + n)
+            total += (n + 31) // 32 * 32            # every input starts on a 128-byte line
+        host = torch.empty(total, dtype=torch.int32, pin_memory=dev.type == "cuda")
+        h = {name: host.numpy()[sl] for name, sl in at.items()}
+        h["rows"].view(np.int64)[:] = rows
+        h["tok"][:] = np.fromiter(itertools.chain.from_iterable(plain(s[0]) for s in seqs), np.int32, qs[-1])
+        h["qs"][:], h["ql"][:], h["kl"][:], h["ks"][:] = qs[:-1], ql, kl, ks[:-1]
+        h["slots"][:] = [s[3] if len(s) > 3 else i for i, s in enumerate(seqs)]
+        bt = h["bt"].reshape(S, self.max_blocks)
+        bt[:] = 0
+        for i, s in enumerate(seqs):
+            new = slice(qs[i], qs[i + 1])
+            h["pos"][new] = np.arange(s[2], kl[i])
+            h["sot"][new] = i
+            bt[i, :len(s[1])] = plain(s[1])
+        on_dev = host.to(dev, non_blocking=True)
+        d = {name: on_dev[sl] for name, sl in at.items()}
+        inp = BatchInputs(token_ids=d["tok"], positions=d["pos"], block_table=d["bt"].view(S, self.max_blocks), seq_lens=d["kl"],
+                          is_prefill=True, seq_of_token=d["sot"], q_start=d["qs"], q_len=d["ql"], max_q_len=max(ql),
+                          logit_rows=d["rows"].view(torch.int64), kv_start=d["ks"],
+                          kv_total=ks[-1], max_cached=max(k - q for k, q in zip(kl, ql)),
+                          slots=d["slots"] if self.stateful else None)
+        i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=dev)      # noqa: E731
         smp = None
         if sampling is not None and any(s[0] > 0 for s in sampling):
             smp = SamplingInputs(torch.tensor([s[0] for s in sampling], dtype=torch.float32, device=dev),
