@@ -47,8 +47,7 @@ class Workspace:
         self.route_barrier = torch.zeros(2, dtype=torch.int32, device=device)
         # Split-KV scratch of decode attention, sized ONCE for the worst case and never reallocated: captured CUDA
         # graphs keep its address, so growing it on demand would leave earlier graphs writing into freed memory.
-        # Splits are only used while (sequences x kv heads x splits) <= SM count (pick_splits) with at most
-        # MAX_GROUP query heads per kv head, which bounds B * Hq * splits; the counters are one per (sequence, kv head).
+        # pick_splits keeps B * Hq * splits within it; the counters are one per (sequence, kv head).
         self.attn_rows_cap = self.sm_count * self.MAX_GROUP
         # A library built for one design may leave the per-head decode kernel out, and its scratch with it.
         floats = int(L.skein_attn_decode_workspace_floats(self.attn_rows_cap, 1, 1)) if hasattr(L, "skein_attn_decode_workspace_floats") else 0
@@ -487,14 +486,18 @@ def rope_kv_append(qkv, positions, seq_of_token, block_table, cos_sin, kv_cache,
     _lib.count_launch()
 
 
-def pick_splits(B, Hkv, ctx_hint, sm_count=148):
-    """Split-KV factor of decode attention: only while there are fewer (sequence, kv head) pairs than SMs, never
-    below 512 tokens per split, never more CTAs than SMs. Each split adds a workspace round trip and a last-arriver
-    merge, which at 64 sequences costs more than the extra parallelism brings."""
+def pick_splits(B, Hkv, ctx_hint, sm_count=148, group=16):
+    """Split-KV factor of decode attention. The kernel is a chain of 16-token tiles per warp, so the longest sequence sets its time until
+    the splits keep every SM at two CTAs (a little more, as sequences are of all lengths); each split adds a workspace round trip and a last-arriver
+    merge, so that it needs more tokens the more (sequence, kv head) pairs there are. Against one CTA per SM and 512 tokens per split, us: 5
+    sequences of up to 8000 tokens x 8 heads 40.2 -> 28.4 (in a batch of 8 rows 54 -> 32), 10 of 4000 54.5 -> 29.8, one of 2000 17.7 -> 13.8, 16 of 4000
+    56.4 -> 43.9; 144 pairs of 512 tokens stay whole (13.8 against 16.7). group: query heads per kv head, for the scratch that the partials
+    share (Workspace.attn_scratch)."""
     if os.environ.get("SKEIN_ATTN_SPLITS"):
         return int(os.environ["SKEIN_ATTN_SPLITS"])
-    ctas = max(B * Hkv, 1)
-    return max(1, min(sm_count // ctas, ctx_hint // 512, 16))
+    pairs = max(B * Hkv, 1)
+    tokens = 256 if pairs <= 40 and ctx_hint >= 768 else 512 if pairs <= 80 else 1000
+    return max(1, min(sm_count * 13 // 6 // pairs, ctx_hint // tokens, sm_count * Workspace.MAX_GROUP // (pairs * group), 16))
 
 
 def _decode_tc_ok(kv_cache, B, Hq, Hkv, D, splits, impl) -> bool:
@@ -528,7 +531,7 @@ def attn_decode(q, kv_cache, block_table, seq_lens, Hq, Hkv, D, scale=None, out=
         out = torch.empty(B, Hq * D, dtype=torch.bfloat16, device=q.device)
     ws = workspace()
     if splits is None:
-        splits = pick_splits(B, Hkv, ctx_hint, ws.sm_count)
+        splits = pick_splits(B, Hkv, ctx_hint, ws.sm_count, Hq // Hkv)
     wsf, ctr = (None, None)
     if splits > 1:
         scratch = ws.attn_scratch(B, Hq, Hkv, splits)
@@ -579,7 +582,7 @@ def attn_decode_rope(qkv, positions, block_table, cos_sin, kv_cache, seq_lens, H
         out = torch.empty(B, Hq * D, dtype=torch.bfloat16, device=qkv.device)
     ws = workspace()
     if splits is None:
-        splits = pick_splits(B, Hkv, ctx_hint, ws.sm_count)
+        splits = pick_splits(B, Hkv, ctx_hint, ws.sm_count, Hq // Hkv)
     wsf, ctr = (None, None)
     if splits > 1:
         scratch = ws.attn_scratch(B, Hq, Hkv, splits)

@@ -174,7 +174,7 @@ def window_attn(q, spec, inp, cache, page_size, out, out_scale=1.0, mix: HeadMix
             page_size, bt.stride(0), cache.shape[0], C.byref(r), _lib.stream_ptr())
     else:
         B, reach = q.shape[0], spec.window + spec.keep_first if spec.window else spec.chunk or inp.ctx_hint
-        splits = F.pick_splits(B, K, min(inp.ctx_hint, reach), ws.sm_count)
+        splits = F.pick_splits(B, K, min(inp.ctx_hint, reach), ws.sm_count, H * spec.maps // K)
         scratch = ws.attn_scratch(B, H * spec.maps, K, splits) if splits > 1 else None
         splits, (wsf, ctr) = (splits, scratch) if scratch is not None else (1, (None, None))
         rc = _lib.lib().skein_attn_decode_window(
