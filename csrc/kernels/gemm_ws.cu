@@ -169,7 +169,10 @@ gemm_ws_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ 
     tma_prefetch_desc(&tmW);
     tma_prefetch_desc(&tmX);
   }
-  pdl_wait();
+  // early: the weights' first tiles are fetched ahead of that wait too, as many as the stages hold (29 MB on the chip); the producer then
+  // waits before the activations, the epilogue before its first store. (Groups take their sizes from the kernel before.)
+  const bool early = p.early_w && p.group_cnt == nullptr && p.group_off == nullptr;
+  if (!early) pdl_wait();
   if (threadIdx.x == 0) build_sched(sched, p, W8 ? 128 : 64, (int)gridDim.x, p.line_cut_only == 0);
   tc_fence_before();
   __syncthreads();
@@ -216,20 +219,7 @@ gemm_ws_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ 
           const bool scales_by_copy = W8 && (w_row + (DUAL ? p.up_row_off : 0) + TILE_F <= w_rows_total) &&
                                       (un.m * TILE_F + TILE_F <= p.F) && (w_rows_total % 4 == 0) && (p.up_row_off % 4 == 0);
           if (W8) tx_bytes = tx_base + (scales_by_copy ? (DUAL ? 2 : 1) * 512u : 0u);
-          for (int kb = kb0; kb < kb1; ++kb, stage.step(a.stages)) {
-            const uint32_t s = stage.i, ph = stage.phase;
-            {
-              PROF_T0();
-              if (!mbar_wait(smem_u32(&bar_empty[s]), ph ^ 1, &abort_flag, a.budget_ns)) {
-                report_status(p.status, ST_TIMEOUT_SMEM_EMPTY, blockIdx.x);
-                abort_flag = 1;
-                ok = false;
-                break;
-              }
-              if (W8) PROF_ADD(5);
-            }
-            const uint32_t full = smem_u32(&bar_full[s]);
-            const uint32_t st = smem_base + s * a.stage_bytes;
+          auto load_w = [&](uint32_t st, uint32_t full, int kb) {
             mbar_expect_tx(full, tx_bytes);
             if (p.w_packed) {
               // tile-packed weights: tile (row tile, kb) is one contiguous 16 KB block
@@ -239,16 +229,35 @@ gemm_ws_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ 
               tma_load_2d(st, &tmW, full, kb * k_elems, w_row, pol_w);
               if (DUAL) tma_load_2d(st + W_TILE_BYTES, &tmW, full, kb * k_elems, w_row + p.up_row_off, pol_w);
             }
+            if (W8 && scales_by_copy) {
+              const float* sp = p.w_scale + (size_t)kb * w_rows_total + w_row;
+              bulk_load_1d(st + a.scale_off, sp, 512, full);
+              if (DUAL) bulk_load_1d(st + a.scale_off + 512, sp + p.up_row_off, 512, full);
+            }
+          };
+          int ahead = 0;       // K-blocks whose weights are on their way already
+          if (early && pos == kb_begin) {
+            for (; ahead < kb1 - kb0 && ahead < a.stages; ++ahead) load_w(smem_base + ahead * a.stage_bytes, smem_u32(&bar_full[ahead]), kb0 + ahead);
+            pdl_wait();
+          }
+          for (int kb = kb0; kb < kb1; ++kb, stage.step(a.stages)) {
+            const uint32_t s = stage.i, ph = stage.phase;
+            const uint32_t full = smem_u32(&bar_full[s]);
+            const uint32_t st = smem_base + s * a.stage_bytes;
+            if (kb - kb0 >= ahead) {
+              PROF_T0();
+              if (!mbar_wait(smem_u32(&bar_empty[s]), ph ^ 1, &abort_flag, a.budget_ns)) {
+                report_status(p.status, ST_TIMEOUT_SMEM_EMPTY, blockIdx.x);
+                abort_flag = 1;
+                ok = false;
+                break;
+              }
+              if (W8) PROF_ADD(5);
+              load_w(st, full, kb);
+            }
             tma_load_2d(st + W_STAGE_BYTES, &tmX, full, x_col + kb * k_elems, x_row, pol_x);
             // e4m3 weights: a stage covers 128 K elements, i.e. two 64-wide bf16 activation tiles
-            if (W8) {
-              tma_load_2d(st + W_STAGE_BYTES + a.x_tile_bytes / 2, &tmX, full, kb * k_elems + 64, x_row, pol_x);
-              if (scales_by_copy) {
-                const float* sp = p.w_scale + (size_t)kb * w_rows_total + w_row;
-                bulk_load_1d(st + a.scale_off, sp, 512, full);
-                if (DUAL) bulk_load_1d(st + a.scale_off + 512, sp + p.up_row_off, 512, full);
-              }
-            }
+            if (W8) tma_load_2d(st + W_STAGE_BYTES + a.x_tile_bytes / 2, &tmX, full, kb * k_elems + 64, x_row, pol_x);
           }
           pos = u * KB + kb1;
         }
@@ -443,6 +452,7 @@ gemm_ws_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ 
       }
     } else if (warp < 6) {
       // ================= epilogue (warps 2..5) =================
+      if (early) pdl_wait();
       const int q = warp & 3;                 // TMEM lane quarter this warp may read
       const int r = q * 32 + lane;            // feature row inside the tile
       const int et = threadIdx.x - 64;        // 0..127
@@ -1035,7 +1045,7 @@ extern "C" int skein_gemm_ws(const SkeinGemmParams* p, void* stream) {
       if (e != cudaSuccess) return e;
       attr_done[variant] = true;
     }
-    return launch_pdl(fn, dim3(grid), dim3(w8 ? W8_THREADS : NUM_THREADS), smem, s, tmW, tmX, ka);
+    return launch_pdl_if(p->early_w != 0 || pdl_enabled(), fn, dim3(grid), dim3(w8 ? W8_THREADS : NUM_THREADS), smem, s, tmW, tmX, ka);
   };
   switch (variant) {
     case 0: return (int)with_kernel(gemm_ws_kernel<false, false>);

@@ -55,7 +55,8 @@ typedef struct SkeinGemmParams {
   int32_t gate_ld;          // elements between rows of gate
   const void* gate;         // optional bf16: the value is multiplied by sigmoid(gate[row, column without out_col0])
   int32_t relu2_cols;       // features below this one are stored as max(y, 0)^2
-  int32_t pad;
+  int32_t early_w;          // 1: neither the kernel before this one in the stream nor one that may still run then writes W or w_scale, so
+                            // that they may be read before it has completed (launched as its programmatic dependent)
 } SkeinGemmParams;
 
 // Returns 0 or a cudaError_t / negative argument-error code.

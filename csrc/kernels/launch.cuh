@@ -9,7 +9,8 @@
 // its first write to memory that an earlier kernel may still read. The attribute is recorded by stream
 // capture, so the overlap is kept inside CUDA graphs.
 //
-// Off unless SKEIN_PDL=1: on the decode step of the flagship model it measured 1-2 % slower than plain
+// Products that may fetch their weights early (gemm_ws.cuh: early_w) are always launched like that: the streaming GEMM's stages fill while the
+// kernel before ends. For the others it is off unless SKEIN_PDL=1: on the decode step of the flagship model it measured 1-2 % slower than plain
 // serialization (132.6 -> 135.1 us per layer at the 8-way tensor-parallel shard shapes). The weight-streaming
 // GEMM needs ~200 KB of shared memory, so its CTAs cannot become resident before the previous kernel's CTAs
 // have left the SM, and the other kernels have no prologue worth overlapping.
@@ -42,7 +43,7 @@ inline int grid_barrier_budget_ms() { static int v = env_ms("SKEIN_GRID_BARRIER_
 inline int gemm_wait_budget_ms() { static int v = env_ms("SKEIN_GEMM_WAIT_MS", 2000); return v; }
 
 template <typename... KArgs, typename... Args>
-inline cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
+inline cudaError_t launch_pdl_if(bool on, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
                               Args&&... args) {
   cudaLaunchConfig_t cfg;
   memset(&cfg, 0, sizeof(cfg));
@@ -52,10 +53,14 @@ inline cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, s
   cfg.stream = stream;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = pdl_enabled() ? 1 : 0;
+  attr[0].val.programmaticStreamSerializationAllowed = on ? 1 : 0;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
   return cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);
+}
+template <typename... KArgs, typename... Args>
+inline cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args&&... args) {
+  return launch_pdl_if(pdl_enabled(), kernel, grid, block, smem, stream, std::forward<Args>(args)...);
 }
 
 }  // namespace skein

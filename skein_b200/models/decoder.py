@@ -547,18 +547,18 @@ class Decoder(LayeredOps, ParallelOps, PrenormOps):
         """Column-parallel (local) projection through the block's bf16 weight or, when the plan's dtype map
         selected fp8 for this block, its block-scaled e4m3 copy."""
         w8 = lw.fp8.get(name)
-        w = getattr(lw, name)
+        w, kept = getattr(lw, name), True      # (kept: the model's own weight; a product may read it before the kernel in front has ended)
         if w8 is not None and self._expand_fp8(x, w8, grouped, rows_hint):
-            w, w8 = w8.dequant(), None
+            w, w8, kept = w8.dequant(), None, False
         if w8 is not None:
             # weights e4m3 with 1 x 128 block scales, activations bf16: the GEMM streams the e4m3 tiles and rescales them
             # to bf16 on their way to the tensor cores (ops/fp8.py)
             if grouped is not None:
-                return fp8.grouped_linear_a16(x, w8, *grouped, swiglu=swiglu, rows_hint=rows_hint)
-            return fp8.linear_a16(x, w8, swiglu=swiglu)
+                return fp8.grouped_linear_a16(x, w8, *grouped, swiglu=swiglu, rows_hint=rows_hint, early_w=True)
+            return fp8.linear_a16(x, w8, swiglu=swiglu, early_w=True)
         if grouped is not None:
-            return ops.grouped_linear(x, w, *grouped, swiglu=swiglu, rows_hint=rows_hint)
-        return ops.swiglu_linear(x, w) if swiglu else ops.linear(x, w)
+            return ops.grouped_linear(x, w, *grouped, swiglu=swiglu, rows_hint=rows_hint, early_w=kept)
+        return ops.swiglu_linear(x, w, early_w=kept) if swiglu else ops.linear(x, w, early_w=kept)
 
     def _expand_fp8(self, x, w8, grouped=None, rows_hint=None) -> bool:
         """Whether an e4m3 weight is expanded to a transient bf16 matrix for this call. The weight-fp8 GEMM rescales a
@@ -588,7 +588,7 @@ class Decoder(LayeredOps, ParallelOps, PrenormOps):
         if w is None:
             w = w8.dequant()      # CPU ranks (reference operators): dequantise, then the bf16 path
         if single:
-            y = ops.grouped_linear(x, w, *grouped) if grouped is not None else ops.linear(x, w)
+            y = ops.grouped_linear(x, w, *grouped, early_w=True) if grouped is not None else ops.linear(x, w, early_w=True)
             return y.unsqueeze(0), None, None
         return self.comm.linear_push(x, w, grouped)
 
@@ -639,7 +639,7 @@ class Decoder(LayeredOps, ParallelOps, PrenormOps):
         """Logits of this rank's vocabulary shard for the rows that need them."""
         if inp.is_prefill and inp.logit_rows is not None:
             normed = normed.index_select(0, inp.logit_rows).contiguous()
-        return ops.linear(normed, self.w.lm_head)
+        return ops.linear(normed, self.w.lm_head, early_w=True)
 
     def forward_logits(self, inp: BatchInputs):
         """A step without sampling: logits of the rows inp.logit_rows (prefill chunks) or of every row."""

@@ -36,7 +36,7 @@ class GemmParams(C.Structure):
         ("wait_budget_ms", C.c_int32), ("w_packed", C.c_int32), ("line_cut_only", C.c_int32),
         ("x_ld", C.c_int32), ("x_group_cols", C.c_int32), ("out_group_cols", C.c_int32), ("glu", C.c_int32),
         ("glu_limit", C.c_float), ("glu_slope", C.c_float), ("out_f32", C.c_int32), ("gate_ld", C.c_int32),
-        ("gate", C.c_void_p), ("relu2_cols", C.c_int32), ("pad", C.c_int32),
+        ("gate", C.c_void_p), ("relu2_cols", C.c_int32), ("early_w", C.c_int32),
     ]
 
 

@@ -201,7 +201,7 @@ def _a16_params(x, w: Fp8Weight, out, F_out, n_tile, mode):
     return p
 
 
-def linear_a16(x, w: Fp8Weight, swiglu: bool = False, out=None, n_tile=None, _cfg=None):
+def linear_a16(x, w: Fp8Weight, swiglu: bool = False, out=None, n_tile=None, _cfg=None, early_w=False):
     """bf16 x [T, K] times a block-scaled e4m3 weight -> bf16 [T, F] (F = rows, or rows / 2 with the SwiGLU pair epilogue)."""
     if not x.is_cuda:
         wd = w.dequant()
@@ -215,12 +215,12 @@ def linear_a16(x, w: Fp8Weight, swiglu: bool = False, out=None, n_tile=None, _cf
     if T == 0:
         return out
     p = _a16_params(x, w, out, Fo, n_tile or _a16_n_tile(T, swiglu), 1 if swiglu else 0)
-    p.w_rows_per_group, p.up_row_off = rows, (Fo if swiglu else 0)
+    p.w_rows_per_group, p.up_row_off, p.early_w = rows, (Fo if swiglu else 0), int(early_w)
     F._gemm_launch(p, "fp8-weight linear", _cfg)
     return out
 
 
-def grouped_linear_a16(xs, w: Fp8Weight, counts, offsets, swiglu: bool = False, out=None, n_tile=None, rows_hint=None, _cfg=None):
+def grouped_linear_a16(xs, w: Fp8Weight, counts, offsets, swiglu: bool = False, out=None, n_tile=None, rows_hint=None, _cfg=None, early_w=False):
     """Per-expert linear over expert-sorted bf16 rows with block-scaled e4m3 expert weights. w.shape = [E, rows, K]."""
     if not xs.is_cuda:
         return ref.grouped_linear(xs, w.dequant(), counts, offsets, swiglu)
@@ -237,7 +237,7 @@ def grouped_linear_a16(xs, w: Fp8Weight, counts, offsets, swiglu: bool = False, 
         n_tile = _a16_n_tile(int(math.ceil(avg * 1.5)), swiglu)
     p = _a16_params(xs, w, out, Fo, n_tile, 1 if swiglu else 0)
     p.G, p.w_rows_per_group, p.up_row_off = E, rows, (Fo if swiglu else 0)
-    p.group_off, p.group_cnt = offsets.data_ptr(), counts.data_ptr()
+    p.group_off, p.group_cnt, p.early_w = offsets.data_ptr(), counts.data_ptr(), int(early_w)
     F._gemm_launch(p, "fp8-weight grouped_linear", _cfg)
     return out
 

@@ -258,10 +258,11 @@ def simt_launch(p: "_lib.GemmParams", x, max_rows: int, what: str):
     _lib.count_launch()
 
 
-def linear(x, w, out=None, residual=None, n_tile=None, _cfg=None, out_f32=False, relu2_cols=0):
+def linear(x, w, out=None, residual=None, n_tile=None, _cfg=None, out_f32=False, relu2_cols=0, early_w=False):
     """y[t, f] = sum_k x[t, k] w[f, k] (+ residual[t, f]). out_f32: the accumulator is stored without rounding to bf16, the
     residual is fp32 too. x may be the first K columns of a wider matrix (rows strided), and out, which may be the residual, a
-    run of columns of one. The first relu2_cols features are stored as max(y, 0)^2."""
+    run of columns of one. The first relu2_cols features are stored as max(y, 0)^2. early_w: the weight is not written by the stream's last
+    kernels (a model's weights), so that the product may begin to fetch it before they have ended."""
     K = w.shape[1]
     if not x.is_cuda:
         y = ref.linear(x[:, :K], w.unpack() if isinstance(w, PackedWeight) else w, residual, out_f32, relu2_cols)
@@ -280,6 +281,7 @@ def linear(x, w, out=None, residual=None, n_tile=None, _cfg=None, out_f32=False,
     wv, _, packed = _wview(w)
     p = _base_params(x, wv, out, F, K, n_tile or pick_n_tile(T, False, F), 0)
     p.w_rows_per_group, p.w_packed, p.out_f32, p.relu2_cols = F, packed, 1 if out_f32 else 0, int(relu2_cols)
+    p.early_w = int(early_w)
     if x.stride(0) != K:
         p.x_ld = x.stride(0)
     if residual is not None:
@@ -303,7 +305,7 @@ def _check_bf16(x):
         raise ValueError("the tensor-core GEMM takes bf16 activations")
 
 
-def swiglu_linear(x, w13, out=None, n_tile=None, _cfg=None, glu=None):
+def swiglu_linear(x, w13, out=None, n_tile=None, _cfg=None, glu=None, early_w=False):
     """silu(x @ w13[:I].T) * (x @ w13[I:].T) with both products from one pass over x; glu (limit, slope): the clamped unit of
     grouped_linear instead."""
     if not x.is_cuda:
@@ -318,7 +320,7 @@ def swiglu_linear(x, w13, out=None, n_tile=None, _cfg=None, glu=None):
     wv, rows_pg, packed = _wview(w13)
     p = _base_params(x, wv, out, inter, K, n_tile or pick_n_tile(T, True), 1)
     p.w_rows_per_group, p.w_packed = rows_pg, packed
-    p.up_row_off = inter
+    p.up_row_off, p.early_w = inter, int(early_w)
     if glu is not None:
         p.glu, p.glu_limit, p.glu_slope = 1, float(glu[0]), float(glu[1])
     if tc_gemm_ok(x, K):
@@ -328,7 +330,7 @@ def swiglu_linear(x, w13, out=None, n_tile=None, _cfg=None, glu=None):
     return out
 
 
-def grouped_linear(xs, w, counts, offsets, swiglu=False, out=None, n_tile=None, rows_hint=None, grid=0, _cfg=None, glu=None):
+def grouped_linear(xs, w, counts, offsets, swiglu=False, out=None, n_tile=None, rows_hint=None, grid=0, _cfg=None, glu=None, early_w=False):
     """Per-expert linear over an expert-sorted activation matrix. glu (limit, slope): the gate/up pair goes through the clamped
     unit min(g, limit) sigmoid(slope g) (clamp(u, +-limit) + 1) instead of silu(g) u.
 
@@ -352,7 +354,7 @@ def grouped_linear(xs, w, counts, offsets, swiglu=False, out=None, n_tile=None, 
         for e0 in range(0, E, _lib.MAX_GROUPS):
             e1 = min(E, e0 + _lib.MAX_GROUPS)
             grouped_linear(xs, w[e0:e1], counts[e0:e1], offsets[e0:e1], swiglu, out, n_tile,
-                           (rows_hint if rows_hint is not None else rows) * (e1 - e0) // E, grid, _cfg, glu)
+                           (rows_hint if rows_hint is not None else rows) * (e1 - e0) // E, grid, _cfg, glu, early_w)
         return out
     avg = (rows_hint if rows_hint is not None else rows) / E
     many = 0 if n_tile or grid else int(avg)
@@ -365,7 +367,7 @@ def grouped_linear(xs, w, counts, offsets, swiglu=False, out=None, n_tile=None, 
     p.up_row_off = F if swiglu else 0
     p.group_off = offsets.data_ptr()
     p.group_cnt = counts.data_ptr()
-    p.grid = grid
+    p.grid, p.early_w = grid, int(early_w)
     if glu is not None:
         p.glu, p.glu_limit, p.glu_slope = 1, float(glu[0]), float(glu[1])
     if tc_gemm_ok(xs, K):
