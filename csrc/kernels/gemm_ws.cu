@@ -139,8 +139,8 @@ gemm_ws_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ 
   const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
 
   // ---- set-up ---------------------------------------------------------------------------------
-  // Nothing before pdl_wait() touches global memory: barriers, TMEM and the descriptor prefetch overlap the
-  // tail of the previous kernel in the stream (launch.cuh).
+  // Before pdl_wait() nothing is touched in global memory but the weights of an early product (below): barriers, TMEM and the descriptor
+  // prefetch overlap the tail of the previous kernel in the stream (launch.cuh).
   pdl_trigger();
   if (threadIdx.x == 0) {
     TS(0);
@@ -170,7 +170,8 @@ gemm_ws_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ 
     tma_prefetch_desc(&tmX);
   }
   // early: the weights' first tiles are fetched ahead of that wait too, as many as the stages hold (29 MB on the chip); the producer then
-  // waits before the activations, the epilogue before its first store. (Groups take their sizes from the kernel before.)
+  // waits before the activations, the epilogue before its first store, the others before their first bounded wait: the kernel before may itself
+  // stand waiting for a peer, for longer than this kernel's budget. (Groups take their sizes from the kernel before.)
   const bool early = p.early_w && p.group_cnt == nullptr && p.group_off == nullptr;
   if (!early) pdl_wait();
   if (threadIdx.x == 0) build_sched(sched, p, W8 ? 128 : 64, (int)gridDim.x, p.line_cut_only == 0);
@@ -265,6 +266,7 @@ gemm_ws_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ 
     } else if (warp == 1) {
       // ================= MMA issuer =================
       if (elect_one()) {
+        if (early) pdl_wait();
         const uint32_t idesc = umma_idesc(1, 1, TILE_F, n_tile);
         Ring stage, slot;
         uint32_t seg = 0;
@@ -361,6 +363,7 @@ gemm_ws_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ 
       // weight row. The raw tile was written by TMA with the 128-byte swizzle (16-byte chunk c of row r sits at chunk
       // c ^ (r & 7)). A warp can reach the tensor-memory lanes 32 * (warp % 4) .. + 31 only, and lane = row of the A operand, so a warp
       // converts the rows of its own lane quarter; 16 K elements become 8 columns.
+      if (early) pdl_wait();
       const int r = (warp & 3) * 32 + lane;
       const uint32_t group = (warp - 6) >> 2;
       const long long w_rows_total = (long long)p.G * p.w_rows_per_group;

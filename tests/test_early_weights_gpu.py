@@ -45,3 +45,32 @@ def test_behind_a_norm(rows, features, K, kind):
     torch.cuda.synchronize()
     ops.workspace().check_status()
     assert torch.equal(eager, want) and torch.equal(got, want)
+
+
+@pytest.mark.parametrize("kind", ["plain", "unit", "e4m3"])
+def test_budget_starts_when_the_kernel_in_front_has_ended(monkeypatch, kind):
+    """A norm that stands waiting for a peer longer than the product's own budget: what is recorded is the peer's flag, not a stage of the product."""
+    from skein_b200.ops import functional as F
+    make = F._base_params
+
+    def short(*args):
+        p = make(*args)
+        p.wait_budget_ms = 20
+        return p
+
+    monkeypatch.setattr(F, "_base_params", short)
+    K, features = 1024, 4096
+    x, gamma = torch.randn(8, K, device=DEV).bfloat16(), torch.ones(K, device=DEV).bfloat16()
+    w = (torch.randn(2 * features, K, device=DEV) * K ** -0.5).bfloat16()
+    q = fp8.quantize_weight(w) if kind == "e4m3" else w
+    part = torch.randn(2, 8, K, device=DEV).bfloat16()
+    flags, epoch = torch.zeros(2, dtype=torch.int32, device=DEV), torch.ones(1, dtype=torch.int32, device=DEV)
+    torch.cuda.synchronize()
+    _, n = ops.reduce_residual_rmsnorm(x, part, gamma, 1e-5, flags=flags, epoch=epoch, wait_budget_ms=300)
+    if kind == "e4m3":
+        fp8.linear_a16(n, q, early_w=True)
+    else:
+        (ops.swiglu_linear if kind == "unit" else ops.linear)(n, q, early_w=True)
+    torch.cuda.synchronize()
+    with pytest.raises(RuntimeError, match="peer flag"):
+        ops.workspace().check_status()
