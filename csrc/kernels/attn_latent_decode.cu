@@ -108,7 +108,6 @@ __global__ void __launch_bounds__(LD_THREADS, 1) attn_latent_decode_kernel(const
   __shared__ uint32_t tmem_slot;
   __shared__ volatile int abort_flag;
   __shared__ int moved;
-  pdl_trigger();
   pdl_wait();
   const int split = blockIdx.x, h0 = blockIdx.y * NH, t = blockIdx.z, ns = p.splits;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -163,6 +162,7 @@ __global__ void __launch_bounds__(LD_THREADS, 1) attn_latent_decode_kernel(const
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  pdl_trigger();      // (not before the allocation: launch.cuh)
   const uint32_t tmem = tmem_slot, tm_o = tmem_slot + 2 * LD_ACC * 32;      // two buffers of S accumulators, then O
 
   if (warp > 0) {

@@ -51,7 +51,6 @@ struct LatentPrefillParams {
 __global__ void __launch_bounds__(LP_THREADS, 1)
 attn_latent_prefill_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                            const __grid_constant__ CUtensorMap tmR, const __grid_constant__ CUtensorMap tmV, const LatentPrefillParams p) {
-  pdl_trigger();
   pdl_wait();
   const int qt = (int)gridDim.x - 1 - (int)blockIdx.x;     // long rows first: the causal work grows with the row
   const int head = blockIdx.y, seq = blockIdx.z;
@@ -92,6 +91,7 @@ attn_latent_prefill_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  pdl_trigger();      // (not before the allocation: launch.cuh)
   const uint32_t tmem = *tmem_slot;
 
   if (warp == 0) {

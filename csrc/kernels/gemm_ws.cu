@@ -141,7 +141,6 @@ gemm_ws_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ 
   // ---- set-up ---------------------------------------------------------------------------------
   // Before pdl_wait() nothing is touched in global memory but the weights of an early product (below): barriers, TMEM and the descriptor
   // prefetch overlap the tail of the previous kernel in the stream (launch.cuh).
-  pdl_trigger();
   if (threadIdx.x == 0) {
     TS(0);
     abort_flag = 0;
@@ -178,6 +177,7 @@ gemm_ws_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ 
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  pdl_trigger();      // (not before the allocation: launch.cuh)
   const uint32_t tmem_base = tmem_base_smem;
   if (threadIdx.x == 0) TS(1);
 

@@ -9,6 +9,9 @@
 // its first write to memory that an earlier kernel may still read. The attribute is recorded by stream
 // capture, so the overlap is kept inside CUDA graphs.
 //
+// A kernel with tensor memory triggers after its allocation, behind a barrier of the CTA. Triggered before it, a CTA of kernel N + 1 on the
+// same SM could take the columns first and hold them until kernel N has completed, which could then not allocate its own: neither would end.
+//
 // Products that may fetch their weights early (gemm_ws.cuh: early_w) are always launched like that: the streaming GEMM's stages fill while the
 // kernel before ends. For the others it is off unless SKEIN_PDL=1: on the decode step of the flagship model it measured 1-2 % slower than plain
 // serialization (132.6 -> 135.1 us per layer at the 8-way tensor-parallel shard shapes). The weight-streaming

@@ -321,11 +321,11 @@ rec_channel_chunk_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_c
     tmem_alloc(smem_u32(tmem_slot), 512);
     tmem_relinquish();
   }
-  pdl_trigger();
   pdl_wait();
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  pdl_trigger();      // (not before the allocation: launch.cuh)
   const uint32_t tm = *tmem_slot;
   const int v_halves = min(2, (p.V - tile0 + 63) / 64);
 
