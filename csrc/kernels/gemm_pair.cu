@@ -232,6 +232,15 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
           tma_load_2d_pair(st + PAIR_W_BYTES, &tmX, full, kb * 64, x_row);
         }
       }
+      // The MMA's commits arrive on both CTAs' barriers: nobody leaves before the last one on every stage is here (a stage never filled passes).
+      for (int i = 0; ok && i < a.stages; ++i, ++it) {
+        const uint32_t s = it % a.stages;
+        if (!mbar_wait(smem_u32(&bar_empty[s]), ((it / a.stages) & 1) ^ 1, &abort_flag, a.budget_ns)) {
+          report_status(p.status, ST_TIMEOUT_SMEM_EMPTY, blockIdx.x);
+          abort_flag = 1;
+          ok = false;
+        }
+      }
     }
   } else if (warp == 1) {
     // ================= MMA issuer of the pair =================

@@ -36,3 +36,13 @@ def test_dependents_are_released_after_tensor_memory_is_allocated(path):
             continue
         trigger = body.index("pdl_trigger()")
         assert alloc < trigger and "__syncthreads()" in body[alloc:trigger]
+
+
+def test_pair_of_ctas_waits_for_every_commit_on_its_stages():
+    """tcgen05.commit arrives on the barriers of both CTAs of a pair; the arrivals of the last round may still be on their way when the work is
+    handed out, so the producer waits for each stage once more behind its loop."""
+    code = _code(KERNELS / "gemm_pair.cu")
+    body = next(b for b in _kernels(code) if "tma_load_2d_pair" in b)
+    producer = body[body.index("if (warp == 0)", body.index("cluster_sync_all")):body.index("} else if (warp == 1)")]
+    behind = producer[producer.rindex("tma_load_2d_pair"):]
+    assert re.search(r"for \(int i = 0; ok && i < a\.stages;.*mbar_wait\(smem_u32\(&bar_empty\[s\]\)", behind, flags=re.S)
