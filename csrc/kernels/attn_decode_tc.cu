@@ -27,6 +27,7 @@
 // Reference: fused_decode_attn (vendor/luminal/crates/luminal_cuda_lite/src/kernel/decode_attention.rs:66-139) and the
 // FlashInfer batch-decode wrapper (vendor/luminal/crates/luminal_cuda_lite/src/host/flashinfer/wrapper.cu:123-251).
 #include "ptx.cuh"
+#include "launch.cuh"
 #include <cuda.h>
 #include <cuda_bf16.h>
 #include <math.h>
@@ -442,13 +443,10 @@ extern "C" int skein_attn_decode_tc(const void* q, long long q_stride, void* kv,
     if (sm_cache[dev] > 0) sms = sm_cache[dev];
   }
   const bool deep = (long long)B * Hkv <= sms;
-  static bool attr_set[2] = {false, false};
-  if (!attr_set[deep ? 1 : 0]) {
-    cudaError_t e = deep ? cudaFuncSetAttribute(attn_decode_tc_kernel<6>, cudaFuncAttributeMaxDynamicSharedMemorySize, DtLayout<6>::SMEM)
-                         : cudaFuncSetAttribute(attn_decode_tc_kernel<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, DtLayout<3>::SMEM);
-    if (e != cudaSuccess) return (int)e;
-    attr_set[deep ? 1 : 0] = true;
-  }
+  static PerDevice deep_allowed, allowed;
+  const cudaError_t e = deep ? allow_smem(deep_allowed, (const void*)attn_decode_tc_kernel<6>, DtLayout<6>::SMEM)
+                             : allow_smem(allowed, (const void*)attn_decode_tc_kernel<3>, DtLayout<3>::SMEM);
+  if (e != cudaSuccess) return (int)e;
   CUtensorMap tmKV;
   int rc = cached_tmap_2d(&tmKV, kv, (uint64_t)num_pages * 2 * Hkv * DT_PS, DT_D, 2, DT_PS);
   if (rc != 0) return rc;

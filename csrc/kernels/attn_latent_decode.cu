@@ -481,12 +481,9 @@ static int latent_decode_launch(const CUtensorMap& tm, LatentDecodeParams& p, in
   if (park > smem) smem = park;
   if (smem > 222 * 1024) return -1;
   auto fn = attn_latent_decode_kernel<NH>;
-  static bool attr_set = false;
-  if (!attr_set) {
-    cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, 222 * 1024);
-    if (e != cudaSuccess) return (int)e;
-    attr_set = true;
-  }
+  static PerDevice allowed;
+  const cudaError_t e = allow_smem(allowed, (const void*)fn, 222 * 1024);
+  if (e != cudaSuccess) return (int)e;
   cudaLaunchConfig_t cfg;
   memset(&cfg, 0, sizeof(cfg));
   cfg.gridDim = dim3(p.splits, groups, T);

@@ -348,12 +348,9 @@ extern "C" int skein_latent_attn_prefill(const void* q, long long q_ld, int q_ro
   if (rc == 0) rc = cached_tmap_2d(&tmR, dense, ctx_rows, L, 2, LP_BN);
   if (rc != 0) return rc;
   const size_t smem = (size_t)(3 * (p.dc + 1) + p.vc) * LP_CHUNK + 1024 + 256;
-  static bool attr_set = false;
-  if (!attr_set) {
-    cudaError_t e = cudaFuncSetAttribute(attn_latent_prefill_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 11 * LP_CHUNK + 1280);
-    if (e != cudaSuccess) return (int)e;
-    attr_set = true;
-  }
+  static PerDevice allowed;
+  const cudaError_t e = allow_smem(allowed, (const void*)attn_latent_prefill_kernel, 11 * LP_CHUNK + 1280);
+  if (e != cudaSuccess) return (int)e;
   const dim3 grid((max_q_len + 2 * LP_BM - 1) / (2 * LP_BM), H, S);
   return (int)launch_pdl(attn_latent_prefill_kernel, grid, dim3(LP_THREADS), smem, (cudaStream_t)stream, tmQ, tmK, tmR, tmV, p);
 }

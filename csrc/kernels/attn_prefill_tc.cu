@@ -34,6 +34,7 @@
 // graph ops (crates/skein_emit/src/op_wiring.rs:2155-2305).
 #include "attn_rule.cuh"
 #include "ptx.cuh"
+#include "launch.cuh"
 #include <cuda.h>
 #include <cuda_bf16.h>
 #include <math.h>
@@ -683,12 +684,9 @@ namespace skein {
 template <int TC_D, bool CAP>
 static int attn_prefill_pair_go(const void* q, long long q_stride, long long q_rows, const void* kv, const AttnPrefillTcParams& p, int S, int max_q_len,
                                 void* stream) {
-  static bool attr_set = false;
-  if (!attr_set) {
-    cudaError_t e = cudaFuncSetAttribute(attn_prefill_pair_kernel<TC_D, CAP>, cudaFuncAttributeMaxDynamicSharedMemorySize, tp_smem(TC_D));
-    if (e != cudaSuccess) return (int)e;
-    attr_set = true;
-  }
+  static PerDevice allowed;
+  const cudaError_t e = allow_smem(allowed, (const void*)attn_prefill_pair_kernel<TC_D, CAP>, tp_smem(TC_D));
+  if (e != cudaSuccess) return (int)e;
   CUtensorMap tmQ, tmKV;
   int rc = cached_tmap_2d(&tmQ, q, (uint64_t)q_rows, (uint64_t)q_stride, 2, TC_BM);
   if (rc != 0) return rc;
@@ -702,12 +700,9 @@ static int attn_prefill_pair_go(const void* q, long long q_stride, long long q_r
 static int attn_prefill_maps_go(const void* q, long long q_stride, long long q_rows, const void* kv, const AttnPrefillTcParams& p, int S, int max_q_len,
                                 void* stream) {
   constexpr int smem = 3 * 2 * TC_HALF_BYTES + 1024 /* alignment slack */ + 256 /* barriers */;
-  static bool attr_set = false;
-  if (!attr_set) {
-    cudaError_t e = cudaFuncSetAttribute(attn_prefill_maps_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e != cudaSuccess) return (int)e;
-    attr_set = true;
-  }
+  static PerDevice allowed;
+  const cudaError_t e = allow_smem(allowed, (const void*)attn_prefill_maps_kernel, smem);
+  if (e != cudaSuccess) return (int)e;
   CUtensorMap tmQ, tmKV;
   int rc = cached_tmap_2d(&tmQ, q, (uint64_t)q_rows, (uint64_t)q_stride, 2, TC_BM / 2);
   if (rc != 0) return rc;

@@ -518,8 +518,10 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
 // CTAs that fit at once, or a negative error: the cut tiles' sums need all of them resident.
 template <bool DUAL>
 static int pair_grid() {
-  static int grid = 0;
-  if (grid == 0) {
+  static PerDevice grid;
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) return -7;
+  return grid.get(dev, [] {
     if (cudaFuncSetAttribute(gemm_pair_kernel<DUAL>, cudaFuncAttributeMaxDynamicSharedMemorySize, PAIR_SMEM_MAX) != cudaSuccess) return -7;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(skein_sm_count() & ~1);
@@ -533,9 +535,8 @@ static int pair_grid() {
     int n = 0;
     if (cudaOccupancyMaxActiveClusters(&n, gemm_pair_kernel<DUAL>, &cfg) != cudaSuccess || n < 1) return -7;
     n = n * 2 < skein_sm_count() ? n * 2 : skein_sm_count() & ~1;
-    grid = n < 148 ? n : 148;       // the workspace and the counters hold this many CTAs' partials
-  }
-  return grid;
+    return n < 148 ? n : 148;       // the workspace and the counters hold this many CTAs' partials
+  });
 }
 
 // Tokens of a tile for `rows` rows: the width for which the rounds of whole and cut tiles cost least, where a K-block of a tile costs the

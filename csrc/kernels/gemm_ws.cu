@@ -1039,15 +1039,12 @@ extern "C" int skein_gemm_ws(const SkeinGemmParams* p, void* stream) {
   rc = cached_tmap_2d_ld(&tmX, p->X, p->x_rows, x_width, p->x_ld > 0 ? p->x_ld : p->K, 2, p->n_tile);
   if (rc) return rc;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  static bool attr_done[4] = {false, false, false, false};
+  static PerDevice allowed[4];
   const bool dual = p->mode == 1;
   const int variant = (w8 ? 2 : 0) + (dual ? 1 : 0);
   auto with_kernel = [&](auto fn) -> cudaError_t {
-    if (!attr_done[variant]) {
-      cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024 - 2048);
-      if (e != cudaSuccess) return e;
-      attr_done[variant] = true;
-    }
+    const cudaError_t e = allow_smem(allowed[variant], (const void*)fn, 227 * 1024 - 2048);
+    if (e != cudaSuccess) return e;
     return launch_pdl_if(p->early_w != 0 || pdl_enabled(), fn, dim3(grid), dim3(w8 ? W8_THREADS : NUM_THREADS), smem, s, tmW, tmX, ka);
   };
   switch (variant) {

@@ -292,12 +292,9 @@ gemm_ws_fp8_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
 
 template <bool DUAL, int NT>
 static int launch_f8(const CUtensorMap& tmW, const CUtensorMap& tmX, const F8Args& ka, int grid, size_t smem, cudaStream_t s) {
-  static bool attr_done = false;
-  if (!attr_done) {
-    cudaError_t e = cudaFuncSetAttribute(gemm_ws_fp8_kernel<DUAL, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024 - 2048);
-    if (e != cudaSuccess) return (int)e;
-    attr_done = true;
-  }
+  static PerDevice allowed;
+  const cudaError_t e = allow_smem(allowed, (const void*)gemm_ws_fp8_kernel<DUAL, NT>, 227 * 1024 - 2048);
+  if (e != cudaSuccess) return (int)e;
   gemm_ws_fp8_kernel<DUAL, NT><<<grid, F8_THREADS, smem, s>>>(tmW, tmX, ka);
   return (int)cudaGetLastError();
 }

@@ -18,6 +18,7 @@
 // GEMM needs ~200 KB of shared memory, so its CTAs cannot become resident before the previous kernel's CTAs
 // have left the SM, and the other kernels have no prologue worth overlapping.
 #pragma once
+#include "per_device.h"
 #include <cuda_runtime.h>
 #include <stdlib.h>
 #include <string.h>
@@ -44,6 +45,18 @@ inline int env_ms(const char* name, int fallback) {
 }
 inline int grid_barrier_budget_ms() { static int v = env_ms("SKEIN_GRID_BARRIER_MS", 2000); return v; }
 inline int gemm_wait_budget_ms() { static int v = env_ms("SKEIN_GEMM_WAIT_MS", 2000); return v; }
+
+// Shared memory beyond 48 KB for a kernel, allowed once on every device that launches it (`done`: static, one per kernel).
+inline cudaError_t allow_smem(PerDevice& done, const void* kernel, int bytes) {
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  const int got = done.get(dev, [&] {
+    e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    return e == cudaSuccess ? 1 : -1;
+  });
+  return got > 0 ? cudaSuccess : e != cudaSuccess ? e : cudaErrorInvalidDevice;
+}
 
 template <typename... KArgs, typename... Args>
 inline cudaError_t launch_pdl_if(bool on, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,

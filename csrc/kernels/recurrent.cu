@@ -343,12 +343,9 @@ static int rec_step_bulk_go(const RecParams& p, const RecGate& g, int B, cudaStr
   int heads = RSB_HEADS;                     // a power of two that divides the heads of a group; enough CTAs before larger ones
   while (heads > 1 && ((p.H / p.G) % heads != 0 || (long long)heads * p.D * p.V * 4 > RSB_MAX || (long long)B * p.H / heads < 444)) heads /= 2;
   const int sm = (heads * p.D * p.V + (RS_WARPS + 1 + heads) * p.V + (2 + (CHANNEL ? heads : 0)) * p.D) * 4;
-  static bool attr_set = false;
-  if (!attr_set) {
-    cudaError_t e = cudaFuncSetAttribute(rec_step_bulk_kernel<T, TAPS, CHANNEL>, cudaFuncAttributeMaxDynamicSharedMemorySize, RSB_MAX + 24 * 1024);
-    if (e != cudaSuccess) return (int)e;
-    attr_set = true;
-  }
+  static PerDevice allowed;
+  const cudaError_t e = allow_smem(allowed, (const void*)rec_step_bulk_kernel<T, TAPS, CHANNEL>, RSB_MAX + 24 * 1024);
+  if (e != cudaSuccess) return (int)e;
   return (int)launch_pdl(rec_step_bulk_kernel<T, TAPS, CHANNEL>, dim3(p.H / heads, B), dim3(RS_THREADS), (size_t)sm, s, p, g, heads);
 }
 

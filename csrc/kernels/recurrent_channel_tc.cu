@@ -559,20 +559,17 @@ static int rec_channel_go(const RecParams& p, const RecChunk& c, int T, int S, c
   __nv_bfloat16* mats = (__nv_bfloat16*)c.chunk_mat;
   __nv_bfloat16* opers = mats + units * 3 * RT_C * RT_C;
   float* factors = (float*)(opers + units * RC_NOPS * RT_C * D);
-  static bool attr_set = false;
-  if (!attr_set) {
-    cudaError_t e = cudaFuncSetAttribute(rec_channel_mats_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, rc_mats_smem(D));
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(rec_channel_chunk_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, rc_smem(D));
-    if (e != cudaSuccess) return (int)e;
-    attr_set = true;
-  }
+  static PerDevice mats_allowed, chunk_allowed;
+  cudaError_t e = allow_smem(mats_allowed, (const void*)rec_channel_mats_kernel<D>, rc_mats_smem(D));
+  if (e == cudaSuccess) e = allow_smem(chunk_allowed, (const void*)rec_channel_chunk_kernel<D>, rc_smem(D));
+  if (e != cudaSuccess) return (int)e;
   CUtensorMap tmX, tmM, tmK;
   int rc = cached_tmap_2d(&tmX, c.qkv, (uint64_t)T, (uint64_t)c.qkv_ld, 2, RT_C);
   if (rc == 0) rc = cached_tmap_2d(&tmM, mats, (uint64_t)units * 3 * RT_C, RT_C, 2, RT_C);
   if (rc == 0) rc = cached_tmap_2d(&tmK, opers, (uint64_t)units * RC_NOPS * RT_C, D, 2, RT_C);
   if (rc != 0) return rc;
   const dim3 g1((c.max_q_len + RT_C - 1) / RT_C, p.H, S), g2((p.V + 127) / 128, p.H, S);
-  cudaError_t e = launch_pdl(rec_channel_mats_kernel<D>, g1, dim3(256), (size_t)rc_mats_smem(D), s, p, c, mats, opers, factors);
+  e = launch_pdl(rec_channel_mats_kernel<D>, g1, dim3(256), (size_t)rc_mats_smem(D), s, p, c, mats, opers, factors);
   if (e != cudaSuccess) return (int)e;
   return (int)launch_pdl(rec_channel_chunk_kernel<D>, g2, dim3(RC_THREADS), (size_t)rc_smem(D), s, tmX, tmM, tmK, p, c, (const float*)factors);
 }

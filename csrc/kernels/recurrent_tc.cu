@@ -501,14 +501,10 @@ static int rec_tc_go(const RecParams& p, const RecChunk& c, int T, int S, cudaSt
   const int units = (T / RT_C + S + 1) * p.H, nmat = DELTA ? 3 : 1;
   __nv_bfloat16* mats = (__nv_bfloat16*)c.chunk_mat;
   float* factors = (float*)(mats + (size_t)units * nmat * RT_C * RT_C);
-  static bool attr_set = false;
-  if (!attr_set) {
-    cudaError_t e = cudaFuncSetAttribute(rec_tc_mats_kernel<D, DELTA>, cudaFuncAttributeMaxDynamicSharedMemorySize, rt_mats_smem(D, DELTA));
-    if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(rec_tc_chunk_kernel<D, DELTA, PAIR>, cudaFuncAttributeMaxDynamicSharedMemorySize, rt_smem(D, DELTA, PAIR));
-    if (e != cudaSuccess) return (int)e;
-    attr_set = true;
-  }
+  static PerDevice mats_allowed, chunk_allowed;
+  cudaError_t e = allow_smem(mats_allowed, (const void*)rec_tc_mats_kernel<D, DELTA>, rt_mats_smem(D, DELTA));
+  if (e == cudaSuccess) e = allow_smem(chunk_allowed, (const void*)rec_tc_chunk_kernel<D, DELTA, PAIR>, rt_smem(D, DELTA, PAIR));
+  if (e != cudaSuccess) return (int)e;
   CUtensorMap tmX, tmM;
   int rc = cached_tmap_2d(&tmX, c.qkv, (uint64_t)T, (uint64_t)c.qkv_ld, 2, RT_C);
   if (rc == 0) rc = cached_tmap_2d(&tmM, mats, (uint64_t)units * nmat * RT_C, RT_C, 2, RT_C);
@@ -516,7 +512,7 @@ static int rec_tc_go(const RecParams& p, const RecChunk& c, int T, int S, cudaSt
   int heads = RT_HB;                            // of a CTA of the first kernel: a power of two that divides the heads of a group
   while ((p.H / p.G) % heads != 0) heads /= 2;
   const dim3 g1((c.max_q_len + RT_C - 1) / RT_C, p.H / heads, S), g2(PAIR ? 1 : (p.V + 127) / 128, PAIR ? p.H / 2 : p.H, S);
-  cudaError_t e = launch_pdl(rec_tc_mats_kernel<D, DELTA>, g1, dim3(256), (size_t)rt_mats_smem(D, DELTA), s, p, c, mats, factors, heads);
+  e = launch_pdl(rec_tc_mats_kernel<D, DELTA>, g1, dim3(256), (size_t)rt_mats_smem(D, DELTA), s, p, c, mats, factors, heads);
   if (e != cudaSuccess) return (int)e;
   return (int)launch_pdl(rec_tc_chunk_kernel<D, DELTA, PAIR>, g2, dim3(RT_THREADS), (size_t)rt_smem(D, DELTA, PAIR), s, tmX, tmM, p, c,
                          (const float*)factors);
