@@ -331,6 +331,12 @@ class Decoder(LayeredOps, ParallelOps, PrenormOps):
     def _multi(self) -> bool:
         return (self.comm is not None and self.comm.size > 1) or (self.comm_moe is not None and self.comm_moe.size > 1)
 
+    @property
+    def _early(self) -> bool:
+        """Whether products of the model's own weights begin to fetch them before the kernel in front has ended. Measured on one rank only; with
+        more, the kernel in front waits for peers, and the product would hold most of every SM's shared memory meanwhile."""
+        return not self._multi
+
     # ---- operators of the program (one method per operator name of the lowering) -----------------------
     def _op_embed_tokens(self, st, _):
         if self.cfg.is_parallel:
@@ -547,18 +553,18 @@ class Decoder(LayeredOps, ParallelOps, PrenormOps):
         """Column-parallel (local) projection through the block's bf16 weight or, when the plan's dtype map
         selected fp8 for this block, its block-scaled e4m3 copy."""
         w8 = lw.fp8.get(name)
-        w, kept = getattr(lw, name), True      # (kept: the model's own weight; a product may read it before the kernel in front has ended)
+        w, early = getattr(lw, name), self._early
         if w8 is not None and self._expand_fp8(x, w8, grouped, rows_hint):
-            w, w8, kept = w8.dequant(), None, False
+            w, w8, early = w8.dequant(), None, False      # (written by the kernel in front)
         if w8 is not None:
             # weights e4m3 with 1 x 128 block scales, activations bf16: the GEMM streams the e4m3 tiles and rescales them
             # to bf16 on their way to the tensor cores (ops/fp8.py)
             if grouped is not None:
-                return fp8.grouped_linear_a16(x, w8, *grouped, swiglu=swiglu, rows_hint=rows_hint, early_w=True)
-            return fp8.linear_a16(x, w8, swiglu=swiglu, early_w=True)
+                return fp8.grouped_linear_a16(x, w8, *grouped, swiglu=swiglu, rows_hint=rows_hint, early_w=early)
+            return fp8.linear_a16(x, w8, swiglu=swiglu, early_w=early)
         if grouped is not None:
-            return ops.grouped_linear(x, w, *grouped, swiglu=swiglu, rows_hint=rows_hint, early_w=kept)
-        return ops.swiglu_linear(x, w, early_w=kept) if swiglu else ops.linear(x, w, early_w=kept)
+            return ops.grouped_linear(x, w, *grouped, swiglu=swiglu, rows_hint=rows_hint, early_w=early)
+        return ops.swiglu_linear(x, w, early_w=early) if swiglu else ops.linear(x, w, early_w=early)
 
     def _expand_fp8(self, x, w8, grouped=None, rows_hint=None) -> bool:
         """Whether an e4m3 weight is expanded to a transient bf16 matrix for this call. The weight-fp8 GEMM rescales a
@@ -572,24 +578,16 @@ class Decoder(LayeredOps, ParallelOps, PrenormOps):
 
     def _row_parallel(self, x, lw, name, grouped=None):
         """Row-parallel projection. Returns (partial [n_src, rows, H], flags, epoch) for the fused reduce."""
-        single = self.comm is None or self.comm.size == 1
+        if self.comm is None or self.comm.size == 1:
+            return self._col_linear(x, lw, name, grouped=grouped).unsqueeze(0), None, None
         w8 = lw.fp8.get(name)
         if w8 is not None and self._expand_fp8(x, w8, grouped):
-            w = w8.dequant()
-            if single:
-                y = ops.grouped_linear(x, w, *grouped) if grouped is not None else ops.linear(x, w)
-                return y.unsqueeze(0), None, None
-            return self.comm.linear_push(x, w, grouped)
-        if w8 is not None and single:
-            return self._col_linear(x, lw, name, grouped=grouped).unsqueeze(0), None, None
+            return self.comm.linear_push(x, w8.dequant(), grouped)
         if w8 is not None and x.is_cuda and hasattr(self.comm, "linear_push_fp8"):
             return self.comm.linear_push_fp8(x, None, w8, grouped)
         w = getattr(lw, name)
         if w is None:
             w = w8.dequant()      # CPU ranks (reference operators): dequantise, then the bf16 path
-        if single:
-            y = ops.grouped_linear(x, w, *grouped, early_w=True) if grouped is not None else ops.linear(x, w, early_w=True)
-            return y.unsqueeze(0), None, None
         return self.comm.linear_push(x, w, grouped)
 
     # ---- the step ---------------------------------------------------------------------------------
@@ -639,7 +637,7 @@ class Decoder(LayeredOps, ParallelOps, PrenormOps):
         """Logits of this rank's vocabulary shard for the rows that need them."""
         if inp.is_prefill and inp.logit_rows is not None:
             normed = normed.index_select(0, inp.logit_rows).contiguous()
-        return ops.linear(normed, self.w.lm_head, early_w=True)
+        return ops.linear(normed, self.w.lm_head, early_w=self._early)
 
     def forward_logits(self, inp: BatchInputs):
         """A step without sampling: logits of the rows inp.logit_rows (prefill chunks) or of every row."""

@@ -61,7 +61,7 @@ class ParallelOps:
     def _op_loop_mix(self, st, li):
         C, w = self.cfg.hidden_size, self.w.loop
         par.residual_tanh(st.residual, dtype=self.act_dtype, out=st.cat[:, :C])
-        y = ops.linear(st.cat, w.w_in, out_f32=True, early_w=True)
+        y = ops.linear(st.cat, w.w_in, out_f32=True, early_w=self._early)
         st.residual, st.normed = par.residual_tanh(None, y, w.step[self.cfg.layers[li].loop_pass], self.w.layers[li].norm, self.act_dtype)
 
     def _op_tanh_norm(self, st, li):
@@ -72,13 +72,13 @@ class ParallelOps:
         lay, T = self.layouts[li], st.residual.shape[0]
         new = torch.zeros if lay.zero_fill else torch.empty
         st.qkv = new(T, lay.width, dtype=self.act_dtype, device=self.device)
-        ops.linear(st.normed, self.w.layers[li].w_in, out=st.qkv[:, lay.in_first:], relu2_cols=lay.ff_cols, early_w=True)
+        ops.linear(st.normed, self.w.layers[li].w_in, out=st.qkv[:, lay.in_first:], relu2_cols=lay.ff_cols, early_w=self._early)
         st.normed = None
 
     def _op_parallel_out(self, st, li):
         lay = self.layouts[li]
         st.residual = ops.linear(st.qkv[:, :lay.out_cols], self.w.layers[li].w_out, out=st.residual, residual=st.residual, out_f32=True,
-                                 early_w=True)
+                                 early_w=self._early)
         st.qkv = None
         if self.capture_hidden is not None:
             self.capture_hidden.append(st.residual.detach().clone().cpu())      # (the next layer adds in place)
