@@ -953,6 +953,7 @@ static int plan(const SkeinGemmParams* p, KernelArgs* ka, int* grid, size_t* sme
   if (p->fp8 == 1) return -6;  // e4m3 x e4m3 with both operands block-scaled goes through skein_gemm_ws_fp8
   if (w8 && (p->w_scale == nullptr || p->w_packed)) return -6;
   ka->p = *p;
+  if (!early_weights_enabled()) ka->p.early_w = 0;
   {
     const int acc_cols = (dual ? 2 : 1) * p->n_tile;
     int st = 32;
@@ -1045,7 +1046,7 @@ extern "C" int skein_gemm_ws(const SkeinGemmParams* p, void* stream) {
   auto with_kernel = [&](auto fn) -> cudaError_t {
     const cudaError_t e = allow_smem(allowed[variant], (const void*)fn, 227 * 1024 - 2048);
     if (e != cudaSuccess) return e;
-    return launch_pdl_if(p->early_w != 0 || pdl_enabled(), fn, dim3(grid), dim3(w8 ? W8_THREADS : NUM_THREADS), smem, s, tmW, tmX, ka);
+    return launch_pdl_if(ka.p.early_w != 0 || pdl_enabled(), fn, dim3(grid), dim3(w8 ? W8_THREADS : NUM_THREADS), smem, s, tmW, tmX, ka);
   };
   switch (variant) {
     case 0: return (int)with_kernel(gemm_ws_kernel<false, false>);

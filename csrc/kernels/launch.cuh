@@ -12,11 +12,11 @@
 // A kernel with tensor memory triggers after its allocation, behind a barrier of the CTA. Triggered before it, a CTA of kernel N + 1 on the
 // same SM could take the columns first and hold them until kernel N has completed, which could then not allocate its own: neither would end.
 //
-// Products that may fetch their weights early (gemm_ws.cuh: early_w) are always launched like that: the streaming GEMM's stages fill while the
-// kernel before ends. For the others it is off unless SKEIN_PDL=1: on the decode step of the flagship model it measured 1-2 % slower than plain
-// serialization (132.6 -> 135.1 us per layer at the 8-way tensor-parallel shard shapes). The weight-streaming
-// GEMM needs ~200 KB of shared memory, so its CTAs cannot become resident before the previous kernel's CTAs
-// have left the SM, and the other kernels have no prologue worth overlapping.
+// Products that may fetch their weights early (gemm_ws.cuh: early_w) are launched like that unless SKEIN_EARLY_WEIGHTS=0: behind a norm or the
+// attention, whose CTAs leave room for theirs (~200 KB of shared memory), the streaming GEMM's stages fill while the kernel before ends (4096 x
+// 4096 in a chain 13.3 -> 11.7 us). For everything else it is off unless SKEIN_PDL=1: on the decode step of the flagship model it measured 1-2 %
+// slower than plain serialization (132.6 -> 135.1 us per layer at the 8-way tensor-parallel shard shapes), as a product cannot become resident behind
+// another one and the other kernels have no prologue worth overlapping.
 #pragma once
 #include "per_device.h"
 #include <cuda_runtime.h>
@@ -26,13 +26,14 @@
 
 namespace skein {
 
+// Read once per process (RuntimeConfig: pdl, early_weights).
 inline bool pdl_enabled() {
-  static int on = -1;
-  if (on < 0) {
-    const char* e = getenv("SKEIN_PDL");
-    on = (e != nullptr && strcmp(e, "1") == 0) ? 1 : 0;
-  }
-  return on == 1;
+  static const bool on = [] { const char* e = getenv("SKEIN_PDL"); return e != nullptr && strcmp(e, "1") == 0; }();
+  return on;
+}
+inline bool early_weights_enabled() {
+  static const bool on = [] { const char* e = getenv("SKEIN_EARLY_WEIGHTS"); return e == nullptr || strcmp(e, "0") != 0; }();
+  return on;
 }
 
 // Wait budgets of the kernels that wait on other CTAs of their own launch, in milliseconds, from the environment

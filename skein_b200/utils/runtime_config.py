@@ -47,6 +47,7 @@ _FIELDS = {
     "gemm_autogrid": ("SKEIN_GEMM_AUTOGRID", _bool, None),
     "pack_moe": ("SKEIN_PACK_MOE", _bool, None),
     "pdl": ("SKEIN_PDL", _bool, None),
+    "early_weights": ("SKEIN_EARLY_WEIGHTS", _bool, None),
     "pp_continuous": ("SKEIN_PP_CONTINUOUS", _bool, None),
     "tune_cache": ("SKEIN_TUNE_CACHE", str, None),
     "grid_barrier_ms": ("SKEIN_GRID_BARRIER_MS", int, None),
@@ -68,7 +69,8 @@ class RuntimeConfig:
     gemm_aligned: bool = True      # tile-aligned K pieces when there are fewer tiles than SMs
     gemm_autogrid: bool = True     # whole tiles per CTA when that wastes little
     pack_moe: bool = True          # tile-packed expert weights
-    pdl: bool = False              # programmatic dependent launch between the per-layer kernels
+    pdl: bool = False              # programmatic dependent launch between all of the per-layer kernels
+    early_weights: bool = True     # products launched so that they fetch the model's weights before the kernel in front has ended
     pp_continuous: bool = False    # pipeline parallelism: one group of sequences per stage in flight across engine steps
     tune_cache: str = ""           # kernel-configuration cache to load ("" = the artifact's own, if any)
     grid_barrier_ms: int = 2000    # budget of the grid-wide arrival counter in the fused reduce + router kernel

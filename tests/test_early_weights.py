@@ -1,4 +1,7 @@
 """Which products may begin to fetch their weights before the kernel in front has ended (early_w)."""
+import os
+import subprocess
+from pathlib import Path
 from types import SimpleNamespace
 
 import pytest
@@ -7,6 +10,9 @@ import torch
 from skein_b200 import ops
 from skein_b200.models.decoder import Decoder
 from skein_b200.ops import fp8
+from skein_b200.utils.runtime_config import RuntimeConfig
+
+ROOT = Path(__file__).resolve().parent.parent
 
 
 class Weight8:
@@ -40,3 +46,18 @@ def test_one_rank_only(monkeypatch, tp, ep, early):
     monkeypatch.setattr(Decoder, "_expand_fp8", lambda *a: True)
     d._col_linear(x, copy8, "wqkv")
     assert seen == [False]
+
+
+def test_switches(tmp_path):
+    """csrc/kernels/launch.cuh: early products have a switch of their own, so that no kernel is a programmatic dependent with both off."""
+    cuda = next((p for p in (Path(os.environ.get("CUDA_HOME", "/usr/local/cuda")),) if (p / "include" / "cuda_runtime.h").exists()), None)
+    if cuda is None:
+        pytest.skip("no CUDA headers")
+    src, exe = tmp_path / "t.cpp", tmp_path / "t"
+    src.write_text('#include "launch.cuh"\n#include <cstdio>\nint main() { printf("%d %d", skein::pdl_enabled(), skein::early_weights_enabled()); }\n')
+    subprocess.run(["g++", "-std=c++17", "-I", str(ROOT / "csrc" / "kernels"), "-I", str(cuda / "include"), str(src), "-o", str(exe)], check=True)
+    base = {k: v for k, v in os.environ.items() if not k.startswith("SKEIN_")}
+    for cfg, want in ((RuntimeConfig(), "0 1"), (RuntimeConfig(early_weights=False), "0 0"), (RuntimeConfig(pdl=True, early_weights=False), "1 0")):
+        assert subprocess.run([str(exe)], env={**base, **cfg.to_env()}, capture_output=True, text=True).stdout == want
+    assert subprocess.run([str(exe)], env=base, capture_output=True, text=True).stdout == "0 1"
+    assert RuntimeConfig.from_toml("[runtime]\nearly_weights = false\n").to_env()["SKEIN_EARLY_WEIGHTS"] == "0"
