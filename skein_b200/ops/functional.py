@@ -128,22 +128,24 @@ def pair_gemm_ok(p: "_lib.GemmParams", rows: int) -> bool:
 
 
 def _gemm_launch(p: "_lib.GemmParams", what: str, cfg: dict | None = None, rows: int = 0):
-    """Launch with (in this order) an explicit configuration of the streaming kernel, the kernel for many rows (rows: of a group, as far as
-    the host knows; 0 keeps a product off it), the measured configuration from the kernel-configuration cache (tuning.py), or the
-    heuristics below."""
+    """Launch with (in this order) an explicit configuration, the measured one from the kernel-configuration cache (tuning.py), or the
+    rules here: pair_gemm_ok for the kernel (rows: of a group, as far as the host knows; 0 keeps a product off the pairs), then the
+    streaming kernel's heuristics below."""
     ws = workspace()
     p.workspace = ws.gemm_ws.data_ptr()
     p.counters = ws.gemm_counters.data_ptr()
     p.status = ws.status.data_ptr()
-    if cfg is None and rows > 0 and pair_gemm_ok(p, rows):
-        _lib.check(_lib.lib().skein_gemm_pair(C.byref(p), _lib.stream_ptr()), what)
-        _lib.count_launch()
-        return
-    p.line_cut_only = 1 if os.environ.get("SKEIN_GEMM_ALIGNED", "1") == "0" else 0
     if cfg is None:
         cache = tuning.active()
         if cache is not None:
             cfg = cache.get("gemm", tuning.gemm_shape_key(p.mode, p.G, p.F, p.K, p.x_rows))
+            if cfg is not None and cfg.get("pair") and p.fp8:      # (measured with bf16 weights of this shape)
+                cfg = None
+    if cfg.get("pair") if cfg is not None else rows > 0 and pair_gemm_ok(p, rows):
+        _lib.check(_lib.lib().skein_gemm_pair(C.byref(p), _lib.stream_ptr()), what)
+        _lib.count_launch()
+        return
+    p.line_cut_only = 1 if os.environ.get("SKEIN_GEMM_ALIGNED", "1") == "0" else 0
     if cfg is not None:
         p.n_tile, p.grid, p.line_cut_only = int(cfg["n_tile"]), int(cfg["grid"]), int(cfg["line_cut_only"])
     elif p.grid == 0 and os.environ.get("SKEIN_GEMM_AUTOGRID", "1") == "1":

@@ -2,7 +2,7 @@
 
 The kernels are compiled ahead of time, so what is left to search at run time is their launch configuration: for the
 weight-streaming GEMM the token-tile width, the grid (whole tiles per CTA or an equal K share per CTA) and the way
-split tiles are cut. `tune_gemm` times the candidates on the device (cold launches inside a CUDA graph, median)
+split tiles are cut; with many rows also whether the kernel on pairs of CTAs takes the product. `tune_gemm` times the candidates on the device (cold launches inside a CUDA graph, median)
 and records the winner; `_gemm_launch` (functional.py) consults the active cache before it falls back to its
 heuristics. Entries are keyed by a hash of the kernel library, so a rebuilt library never reuses stale winners. The
 compile pipeline stores the file as `cache/kernel_configs.json` inside the artifact and `serve` loads it.
@@ -167,11 +167,21 @@ def gemm_candidates(mode: int, G: int, F: int, rows: int, sm_count: int):
     return out
 
 
+PAIR_TUNE_ROWS = 64     # rows of a group from which the kernel on pairs of CTAs is worth timing
+
+
+def pair_candidate(mode: int, G: int, F: int, K: int, rows: int) -> list:
+    """The kernel on pairs of CTAs (csrc/kernels/gemm_pair.cu), which chooses its tiles itself: one configuration, or none where it has no use."""
+    if mode > 1 or rows // max(G, 1) < PAIR_TUNE_ROWS or F < 256 or K < 256:
+        return []
+    return [{"pair": 1, "n_tile": 128, "grid": 0, "line_cut_only": 0}]
+
+
 def tune_gemm(run, mode: int, G: int, F: int, K: int, rows: int, cache: KernelConfigCache | None = None, iters: int = 9,
               budget: int = 0):
     """Time `run(config)` (one launch of the GEMM with that configuration) for every candidate and record the fastest.
 
-    run: callable taking a dict {"n_tile", "grid", "line_cut_only"}; it must launch on the current stream. Returns
+    run: callable taking a dict {"n_tile", "grid", "line_cut_only"[, "pair"]}; it must launch on the current stream. Returns
     (best_config, {config_json: median_us}). `budget` > 0 caps the number of candidates that are timed."""
     import torch
     from .functional import workspace
@@ -179,7 +189,7 @@ def tune_gemm(run, mode: int, G: int, F: int, K: int, rows: int, cache: KernelCo
     flush = torch.empty(256 << 20, dtype=torch.uint8, device="cuda")
     results = {}
     best, best_us = None, float("inf")
-    candidates = gemm_candidates(mode, G, F, rows, workspace().sm_count)
+    candidates = pair_candidate(mode, G, F, K, rows) + gemm_candidates(mode, G, F, rows, workspace().sm_count)
     if budget > 0:
         candidates = candidates[:budget]
     for cfg in candidates:

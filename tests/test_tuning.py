@@ -91,3 +91,50 @@ def test_heuristic_grid_whole_tiles_only_when_they_waste_little():
     assert tuning.heuristic_grid(224, 64, 148) == 0        # 31 idle K-blocks per CTA ...
     assert tuning.heuristic_grid(224, 64, 148, dual=True) == 112   # ... but the two-accumulator kernel keeps whole tiles
     assert tuning.heuristic_grid(100, 64, 148) == 0 and tuning.heuristic_grid(896, 64, 148) == 0   # outside (SMs, 2 SMs]
+
+
+def test_pair_candidate_where_it_has_a_use():
+    assert tuning.pair_candidate(0, 1, 6144, 4096, 512) and tuning.pair_candidate(1, 8, 14336, 4096, 1024)
+    for mode, G, F, K, rows in ((2, 1, 6144, 4096, 512), (0, 1, 6144, 4096, 63), (0, 8, 4096, 14336, 500), (0, 1, 128, 4096, 512), (0, 1, 4096, 128, 512)):
+        assert tuning.pair_candidate(mode, G, F, K, rows) == []
+    assert {"n_tile", "grid", "line_cut_only"} <= set(tuning.pair_candidate(0, 1, 4096, 4096, 64)[0])      # what readers of an entry expect
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("kind", ["linear", "unit", "groups"])
+def test_a_measured_configuration_decides_over_the_rules(monkeypatch, kind):
+    """Both ways: a streaming configuration where the rules would take pairs of CTAs, and pairs where they would not; and with the tuner's own winner."""
+    from skein_b200 import ops
+    from skein_b200.ops import _lib
+    g = torch.Generator(device="cuda").manual_seed(0)
+    rows, F, K, G = 1024, 4096, 4096, 2 if kind == "groups" else 1
+    x = torch.randn(rows, K, device="cuda", generator=g).bfloat16()
+    w = (torch.randn(*((G,) if G > 1 else ()), F * (2 if kind == "unit" else 1), K, device="cuda", generator=g) / 64).bfloat16()
+    cnt = torch.tensor([600, 424], dtype=torch.int32, device="cuda")
+    off = torch.cat([cnt.new_zeros(1), cnt.cumsum(0).int()])
+    call = {"linear": lambda: ops.linear(x, w), "unit": lambda: ops.swiglu_linear(x, w), "groups": lambda: ops.grouped_linear(x, w, cnt, off)}[kind]
+    want = call().float()
+    key = tuning.gemm_shape_key(1 if kind == "unit" else 0, G, F, K, rows)
+    lib = _lib.lib()
+    try:
+        for pair, other in ((0, "skein_gemm_pair"), (1, "skein_gemm_ws")):
+            cache = tuning.KernelConfigCache()
+            cache.put("gemm", key, {"n_tile": 64, "grid": 0, "line_cut_only": 0, **({"pair": 1} if pair else {})})
+            tuning.activate(cache)
+            with monkeypatch.context() as m:
+                m.setattr(lib, other, None)      # must not be the one that runs
+                got = call()
+            torch.cuda.synchronize()
+            ops.workspace().check_status()
+            assert float((got.float() - want).abs().max()) < 2e-2 * float(want.abs().max())
+        cache = tuning.KernelConfigCache()
+        tuning.activate(cache)
+        best, results = ops.tune_grouped(x, w, cnt, off, cache=cache) if kind == "groups" else ops.tune_linear(x, w, swiglu=kind == "unit", cache=cache)
+        assert any(json.loads(c).get("pair") for c in results) and any(not json.loads(c).get("pair") for c in results)
+        with monkeypatch.context() as m:
+            m.setattr(lib, "skein_gemm_ws" if best.get("pair") else "skein_gemm_pair", None)
+            call()
+        torch.cuda.synchronize()
+        ops.workspace().check_status()
+    finally:
+        tuning.activate(None)
