@@ -6,13 +6,16 @@
 // 16 + 16 mma.sync m16n8k16 instead of ~4k scalar FMAs per warp, and K/V tiles stream from the
 // cache into shared memory with cp.async while earlier tiles are being multiplied.
 //
-//   grid = (splits, Hkv, B), 128 threads. The split's range of 16-token tiles is dealt round-robin
+//   grid = (Hkv, B, splits), 128 threads. The split's range of 16-token tiles is dealt round-robin
 //   to the 4 warps. Each warp runs its own 3- or 6-stage pipeline (no CTA-wide barrier in the loop):
 //       cp.async tile i+2 (K 4 KB + V 4 KB, XOR-swizzled rows)      wait tile i
 //       S = Q K^T  (2 n-tiles x 8 k-steps)   online softmax in registers   O += P V (16 n-tiles)
 //   and keeps (m, l, O) for its share of the tokens. The warps' states are merged through shared
 //   memory; with splits > 1 the CTA parks its state in a workspace and the last CTA of a
-//   (sequence, kv head) to arrive merges the splits, as in the scalar kernel.
+//   (sequence, kv head) to arrive merges the splits, as in the scalar kernel. The host knows the batch's context
+//   only as a bound (a server passes the largest it serves): a sequence takes as many of the splits as its own length
+//   is worth, one per split_tokens (a power of two), and the other CTAs leave at once. 10 sequences of 100 tokens x 8 heads under a bound of 8192:
+//   18 us with all four splits, 9 with one.
 //
 // Under a rule (SkeinAttnRule) the tiles are those of the window and, in front of them, those of the first tokens that it keeps in sight.
 //
@@ -55,6 +58,7 @@ struct AttnMmaParams {
   int* status;
   long long q_stride;
   int B, Hq, Hkv, G, page_size, max_blocks, num_pages, splits;   // Hq, G: query rows, the maps of differential heads counted apart
+  int split_log2;                                                 // log2 of the tokens that make a split worth its merge (0: every split is used)
   float scale_log2e, cap_in, cap_log2e;      // (cap_log2e 0: scores are not capped; attn_cap)
   // optional fusion of RoPE and the KV append of the new token (cos_sin == nullptr: q is already rotated and
   // the cache already holds the token). q then points at the raw fused q/k/v projection rows
@@ -104,7 +108,7 @@ __global__ void __launch_bounds__(AM_THREADS) attn_decode_mma_kernel(const AttnM
   __shared__ int is_last;
   pdl_trigger();
   pdl_wait();   // q, the cache and the sequence lengths come from earlier kernels of the step
-  const int split = blockIdx.x, kvh = blockIdx.y, b = blockIdx.z;
+  const int split = blockIdx.z, kvh = blockIdx.x, b = blockIdx.y;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int G = p.G, ps = p.page_size;
   const int len = p.seq_lens[b];
@@ -115,7 +119,8 @@ __global__ void __launch_bounds__(AM_THREADS) attn_decode_mma_kernel(const AttnM
   const int keep = p.r.keep_first, tile_lo = lo / AM_TILE, unit = p.r.window > 0 || p.r.chunk > 0 ? AM_TILE : ps;
   const int kept = min((keep + AM_TILE - 1) / AM_TILE, tile_lo), hop = tile_lo - kept;     // tiles of the first tokens; skipped behind them
   const int row_len = len - hop * AM_TILE;
-  int per = (row_len + p.splits - 1) / p.splits;
+  const int ns = p.split_log2 > 0 ? max(1, min(p.splits, (row_len + (1 << (p.split_log2 - 1))) >> p.split_log2)) : p.splits;
+  int per = (row_len + ns - 1) / ns;
   per = (per + unit - 1) / unit * unit;
   const int t_begin = split * per, t_end = min(t_begin + per, row_len);
   const int tile_begin = t_begin / AM_TILE;
@@ -168,7 +173,7 @@ __global__ void __launch_bounds__(AM_THREADS) attn_decode_mma_kernel(const AttnM
     // the barrier below orders these stores before the asynchronous copies that read them back
     if (pos >= 0) {
       int s_app = per > 0 ? pos / per : 0;
-      if (s_app > p.splits - 1) s_app = p.splits - 1;
+      if (s_app > ns - 1) s_app = ns - 1;
       if (s_app == split) {
         int pg = p.block_table[(size_t)b * p.max_blocks + pos / ps];
         if (pg < 0 || pg >= p.num_pages) {
@@ -191,6 +196,7 @@ __global__ void __launch_bounds__(AM_THREADS) attn_decode_mma_kernel(const AttnM
       }
     }
   }
+  if (split >= ns) return;      // (here, so that the queries' loads do not wait for the length's)
   __syncthreads();
   uint32_t qf[KS][4];
 #pragma unroll
@@ -386,7 +392,7 @@ __global__ void __launch_bounds__(AM_THREADS) attn_decode_mma_kernel(const AttnM
       O_g[g] = O; M_g[g] = M; L_g[g] = L;
     }
   }
-  if (p.splits == 1) {
+  if (ns == 1) {
     if (AM_D == AM_THREADS && p.r.maps == 2) {
       store_pairs([&](int g) { return O_g[g] * attn_norm(M_g[g], L_g[g], sink_of(g)); });
       return;
@@ -409,13 +415,13 @@ __global__ void __launch_bounds__(AM_THREADS) attn_decode_mma_kernel(const AttnM
   if (tid == 0) {
     int* ctr = p.counters + b * p.Hkv + kvh;
     const int old = atomicAdd(ctr, 1);
-    is_last = (old == p.splits - 1);
+    is_last = (old == ns - 1);
     if (is_last) *ctr = 0;
   }
   __syncthreads();
   if (!is_last) return;
   __threadfence();
-  // last CTA of this (sequence, kv head): merge the splits. (m, l) of all heads and splits are staged in
+  // last CTA of this (sequence, kv head): merge the splits in use. (m, l) of all heads and splits are staged in
   // shared memory with one parallel load; each thread then fetches its dim of all splits at once.
   float* ml_s = reinterpret_cast<float*>(am_smem);   // [G][splits][2]
   float* val_s = ml_s + 16 * AM_MAX_SPLITS * 2;      // [G][AM_D], two maps
@@ -426,13 +432,13 @@ __global__ void __launch_bounds__(AM_THREADS) attn_decode_mma_kernel(const AttnM
     const size_t base = base0 + (size_t)g * p.splits;
     float ov[AM_MAX_SPLITS];
 #pragma unroll
-    for (int s2 = 0; s2 < AM_MAX_SPLITS; ++s2) ov[s2] = (s2 < p.splits) ? __ldcg(&p.ws_o[(base + s2) * AM_D + d]) : 0.f;
+    for (int s2 = 0; s2 < AM_MAX_SPLITS; ++s2) ov[s2] = (s2 < ns) ? __ldcg(&p.ws_o[(base + s2) * AM_D + d]) : 0.f;
     float M = -INFINITY;
-    for (int s2 = 0; s2 < p.splits; ++s2) M = fmaxf(M, ml_s[(g * p.splits + s2) * 2]);
+    for (int s2 = 0; s2 < ns; ++s2) M = fmaxf(M, ml_s[(g * p.splits + s2) * 2]);
     float L = 0.f, O = 0.f;
 #pragma unroll
     for (int s2 = 0; s2 < AM_MAX_SPLITS; ++s2) {
-      if (s2 < p.splits) {
+      if (s2 < ns) {
         const float mi = ml_s[(g * p.splits + s2) * 2];
         const float w = (mi == -INFINITY) ? 0.f : exp2f(mi - M);
         L += w * ml_s[(g * p.splits + s2) * 2 + 1];
@@ -464,7 +470,7 @@ static int attn_decode_mma_go(AttnMmaParams& p, float* ws, void* stream) {
   }
   p.ws_o = ws;
   p.ws_ml = ws ? ws + (size_t)p.B * p.Hq * p.splits * AM_D : nullptr;
-  dim3 grid(p.splits, p.Hkv, p.B);
+  const dim3 grid(p.Hkv, p.B, p.splits);      // (splits last: those that leave at once must not take half of the SMs from the others)
   int sms = 0;
   if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0) sms = 148;
   if ((long long)p.splits * p.Hkv * p.B <= sms)
@@ -474,11 +480,11 @@ static int attn_decode_mma_go(AttnMmaParams& p, float* ws, void* stream) {
 
 }  // namespace skein
 
-// Same contract as skein_attn_decode (ws / counters from skein_attn_decode_workspace_floats; counters zero at
+// split_tokens: tokens that make a split worth its merge, a power of two, or 0 where every split is used. Otherwise the same contract as skein_attn_decode (ws / counters from skein_attn_decode_workspace_floats; counters zero at
 // first use). Requires D = 128 (64 without RoPE fusion), page_size a multiple of 16, at most 16 query heads per kv head.
 static int attn_decode_mma_launch(const void* q, long long q_stride, void* kv, const int* block_table,
                                   const int* seq_lens, void* out, long long out_ld, float* ws, int* counters, int* status, int B,
-                                  int Hq, int Hkv, int D, int page_size, int max_blocks, int num_pages, int splits, const SkeinAttnRule& rule,
+                                  int Hq, int Hkv, int D, int page_size, int max_blocks, int num_pages, int splits, int split_tokens, const SkeinAttnRule& rule,
                                   const float* cos_sin, const int* positions, int max_pos, void* stream) {
   using namespace skein;
   if (B == 0) return 0;
@@ -487,7 +493,7 @@ static int attn_decode_mma_launch(const void* q, long long q_stride, void* kv, c
   if ((D != 128 && (D != 64 || cos_sin != nullptr)) || Hq % Hkv != 0 || page_size % AM_TILE != 0) return -1;
   const int G = Hq / Hkv;
   if (G > 16 || q_stride % 8 != 0 || (uintptr_t)q % 16 != 0 || ((rule.window > 0 || rule.chunk > 0) && cos_sin != nullptr)) return -1;
-  if (splits < 1 || splits > AM_MAX_SPLITS) return -2;
+  if (splits < 1 || splits > AM_MAX_SPLITS || split_tokens < 0 || split_tokens == 1 || (split_tokens & (split_tokens - 1)) != 0) return -2;
   if (splits > 1 && (ws == nullptr || counters == nullptr)) return -2;
   AttnMmaParams p;
   p.q = (const __nv_bfloat16*)q; p.kv = (const __nv_bfloat16*)kv; p.kv_rw = (__nv_bfloat16*)kv;
@@ -496,7 +502,7 @@ static int attn_decode_mma_launch(const void* q, long long q_stride, void* kv, c
   p.out = (__nv_bfloat16*)out; p.out_ld = out_ld; p.r = rule;
   p.counters = counters; p.status = status; p.q_stride = q_stride;
   p.B = B; p.Hq = Hq; p.Hkv = Hkv; p.G = G; p.page_size = page_size; p.max_blocks = max_blocks; p.num_pages = num_pages;
-  p.splits = splits; p.scale_log2e = rule.scale * 1.4426950408889634f;
+  p.splits = splits; p.split_log2 = split_tokens > 0 ? 31 - __builtin_clz(split_tokens) : 0; p.scale_log2e = rule.scale * 1.4426950408889634f;
   p.cap_log2e = rule.softcap * 1.4426950408889634f;
   p.cap_in = rule.softcap > 0.f ? 2.f * p.scale_log2e / rule.softcap : 0.f;
   return D == 64 ? attn_decode_mma_go<64>(p, ws, stream) : attn_decode_mma_go<128>(p, ws, stream);
@@ -510,19 +516,19 @@ static SkeinAttnRule plain_rule(float scale) {
 
 extern "C" int skein_attn_decode_mma(const void* q, long long q_stride, const void* kv, const int* block_table,
                                      const int* seq_lens, void* out, float* ws, int* counters, int* status, int B,
-                                     int Hq, int Hkv, int D, int page_size, int max_blocks, int num_pages, int splits,
+                                     int Hq, int Hkv, int D, int page_size, int max_blocks, int num_pages, int splits, int split_tokens,
                                      float scale, void* stream) {
   return attn_decode_mma_launch(q, q_stride, const_cast<void*>(kv), block_table, seq_lens, out, (long long)Hq * D, ws, counters, status, B,
-                                Hq, Hkv, D, page_size, max_blocks, num_pages, splits, plain_rule(scale), nullptr, nullptr, 0, stream);
+                                Hq, Hkv, D, page_size, max_blocks, num_pages, splits, split_tokens, plain_rule(scale), nullptr, nullptr, 0, stream);
 }
 
 // The same under a rule (attn_rule.cuh), into rows out_ld apart. D is the width of a key head; with two maps it must be 128.
 extern "C" int skein_attn_decode_window(const void* q, long long q_stride, const void* kv, const int* block_table,
                                         const int* seq_lens, void* out, long long out_ld, float* ws, int* counters, int* status, int B,
-                                        int Hq, int Hkv, int D, int page_size, int max_blocks, int num_pages, int splits,
+                                        int Hq, int Hkv, int D, int page_size, int max_blocks, int num_pages, int splits, int split_tokens,
                                         const SkeinAttnRule* rule, void* stream) {
   return attn_decode_mma_launch(q, q_stride, const_cast<void*>(kv), block_table, seq_lens, out, out_ld, ws, counters, status, B, Hq, Hkv, D,
-                                page_size, max_blocks, num_pages, splits, *rule, nullptr, nullptr, 0, stream);
+                                page_size, max_blocks, num_pages, splits, split_tokens, *rule, nullptr, nullptr, 0, stream);
 }
 
 // Decode attention straight from the fused q/k/v projection: rotates q and k (rotate-half RoPE from the fp32
@@ -532,9 +538,9 @@ extern "C" int skein_attn_decode_window(const void* q, long long q_stride, const
 extern "C" int skein_attn_decode_rope_mma(const void* qkv, long long qkv_stride, void* kv, const int* block_table,
                                           const int* seq_lens, const int* positions, const float* cos_sin,
                                           int max_pos, void* out, float* ws, int* counters, int* status, int B, int Hq,
-                                          int Hkv, int D, int page_size, int max_blocks, int num_pages, int splits,
+                                          int Hkv, int D, int page_size, int max_blocks, int num_pages, int splits, int split_tokens,
                                           float scale, void* stream) {
   if (cos_sin == nullptr || positions == nullptr) return -1;
   return attn_decode_mma_launch(qkv, qkv_stride, kv, block_table, seq_lens, out, (long long)Hq * D, ws, counters, status, B, Hq, Hkv, D,
-                                page_size, max_blocks, num_pages, splits, plain_rule(scale), cos_sin, positions, max_pos, stream);
+                                page_size, max_blocks, num_pages, splits, split_tokens, plain_rule(scale), cos_sin, positions, max_pos, stream);
 }

@@ -148,9 +148,9 @@ def lib():
     _sig(L, "skein_attn_decode", i32,
          [vp, i64, vp, vp, vp, vp, vp, vp, vp, i32, i32, i32, i32, i32, i32, i32, i32, f32, vp])
     _sig(L, "skein_attn_decode_mma", i32,
-         [vp, i64, vp, vp, vp, vp, vp, vp, vp, i32, i32, i32, i32, i32, i32, i32, i32, f32, vp])
+         [vp, i64, vp, vp, vp, vp, vp, vp, vp, i32, i32, i32, i32, i32, i32, i32, i32, i32, f32, vp])
     _sig(L, "skein_attn_decode_rope_mma", i32,
-         [vp, i64, vp, vp, vp, vp, vp, i32, vp, vp, vp, vp, i32, i32, i32, i32, i32, i32, i32, i32, f32, vp])
+         [vp, i64, vp, vp, vp, vp, vp, i32, vp, vp, vp, vp, i32, i32, i32, i32, i32, i32, i32, i32, i32, f32, vp])
     _sig(L, "skein_attn_prefill", i32,
          [vp, i64, vp, vp, vp, vp, vp, vp, vp, i32, i32, i32, i32, i32, i32, i32, i32, f32, vp])
     _sig(L, "skein_attn_decode_tc", i32,
@@ -211,7 +211,7 @@ def lib():
     arule = C.POINTER(AttnRule)
     _sig(L, "skein_window_attn_rows", i32, [vp, i64, vp, vp, vp, vp, vp, i64, vp, i32, i32, i32, i32, i32, i32, i32, i32, arule, i32, vp])
     _sig(L, "skein_attn_decode_window", i32,
-         [vp, i64, vp, vp, vp, vp, i64, vp, vp, vp, i32, i32, i32, i32, i32, i32, i32, i32, arule, vp])
+         [vp, i64, vp, vp, vp, vp, i64, vp, vp, vp, i32, i32, i32, i32, i32, i32, i32, i32, i32, arule, vp])
     _sig(L, "skein_attn_prefill_window", i32,
          [vp, i64, i64, vp, vp, vp, vp, vp, vp, i64, vp, i32, i32, i32, i32, i32, i32, i32, i32, arule, vp])
     scanp = C.POINTER(ScanParams)

@@ -47,7 +47,7 @@ class Workspace:
         self.route_barrier = torch.zeros(2, dtype=torch.int32, device=device)
         # Split-KV scratch of decode attention, sized ONCE for the worst case and never reallocated: captured CUDA
         # graphs keep its address, so growing it on demand would leave earlier graphs writing into freed memory.
-        # pick_splits keeps B * Hq * splits within it; the counters are one per (sequence, kv head).
+        # split_plan keeps B * Hq * splits within it; the counters are one per (sequence, kv head).
         self.attn_rows_cap = self.sm_count * self.MAX_GROUP
         # A library built for one design may leave the per-head decode kernel out, and its scratch with it.
         floats = int(L.skein_attn_decode_workspace_floats(self.attn_rows_cap, 1, 1)) if hasattr(L, "skein_attn_decode_workspace_floats") else 0
@@ -490,18 +490,33 @@ def rope_kv_append(qkv, positions, seq_of_token, block_table, cos_sin, kv_cache,
     _lib.count_launch()
 
 
+def split_plan(B, Hkv, ctx_hint, sm_count=148, group=16):
+    """(splits, tokens that make a split worth its merge, a power of two) of decode attention on the mma.sync kernel, a chain of 16-token tiles per warp, for contexts
+    of up to ctx_hint tokens; a sequence takes one split per so many tokens of its own. As many as put one CTA on every SM where that is six and
+    more (16 pairs of (sequence, kv head) at 4096 tokens: 19.9 us with 8, 20.9 with 16), else two CTAs per SM and never more, as a third one waits
+    for the others to end (32 pairs of 8000 tokens: 38.5 us with 8, 51.8 with 10; 160 pairs of 2048: 44 whole, 60 in two). A split adds a workspace
+    round trip and a merge, so that it needs more tokens the more pairs there are: with 113 to 148 pairs two splits cost 2 to 7 % for
+    sequences of one length below 8000 tokens. Against one CTA per SM and 512 tokens per split, us, one length / lengths from a fifth up:
+    40 pairs of 8000 47.7 / 42.3 -> 45.2 / 33.0, of 1024 17.3 / 16.2 -> 16.8 / 14.7; 80 of 4096 58.7 / 55.5 -> 45.1 / 36.7; 8 of 768 16.8 -> 14.0.
+    group: query heads per kv head, for the scratch that the partials share (Workspace.attn_scratch)."""
+    if os.environ.get("SKEIN_ATTN_SPLITS"):
+        return int(os.environ["SKEIN_ATTN_SPLITS"]), 0
+    pairs = max(B * Hkv, 1)
+    one = sm_count // pairs
+    tokens = 256 if pairs <= 40 and ctx_hint >= 768 else 512 if pairs <= 80 else 1000 if pairs <= 112 else 4000
+    fit = one if one >= 6 else 2 * sm_count // pairs
+    return max(1, min(fit, ctx_hint // tokens, sm_count * Workspace.MAX_GROUP // (pairs * group), 16)), 1 << round(math.log2(tokens))
+
+
 def pick_splits(B, Hkv, ctx_hint, sm_count=148, group=16):
-    """Split-KV factor of decode attention. The kernel is a chain of 16-token tiles per warp, so the longest sequence sets its time until
-    the splits keep every SM at two CTAs (a little more, as sequences are of all lengths); each split adds a workspace round trip and a last-arriver
-    merge, so that it needs more tokens the more (sequence, kv head) pairs there are. Against one CTA per SM and 512 tokens per split, us: 5
-    sequences of up to 8000 tokens x 8 heads 40.2 -> 28.4 (in a batch of 8 rows 54 -> 32), 10 of 4000 54.5 -> 29.8, one of 2000 17.7 -> 13.8, 16 of 4000
-    56.4 -> 43.9; 144 pairs of 512 tokens stay whole (13.8 against 16.7). group: query heads per kv head, for the scratch that the partials
-    share (Workspace.attn_scratch)."""
+    return split_plan(B, Hkv, ctx_hint, sm_count, group)[0]
+
+
+def _scalar_splits(B, Hkv, ctx_hint, sm_count):
+    """Of the FMA kernel, which uses every split whatever a sequence's length: one CTA per SM at most, 512 tokens of the hint each."""
     if os.environ.get("SKEIN_ATTN_SPLITS"):
         return int(os.environ["SKEIN_ATTN_SPLITS"])
-    pairs = max(B * Hkv, 1)
-    tokens = 256 if pairs <= 40 and ctx_hint >= 768 else 512 if pairs <= 80 else 1000
-    return max(1, min(sm_count * 13 // 6 // pairs, ctx_hint // tokens, sm_count * Workspace.MAX_GROUP // (pairs * group), 16))
+    return max(1, min(sm_count // max(B * Hkv, 1), ctx_hint // 512, 16))
 
 
 def _decode_tc_ok(kv_cache, B, Hq, Hkv, D, splits, impl) -> bool:
@@ -534,8 +549,16 @@ def attn_decode(q, kv_cache, block_table, seq_lens, Hq, Hkv, D, scale=None, out=
     if out is None:
         out = torch.empty(B, Hq * D, dtype=torch.bfloat16, device=q.device)
     ws = workspace()
-    if splits is None:
-        splits = pick_splits(B, Hkv, ctx_hint, ws.sm_count, Hq // Hkv)
+    kernel = impl or os.environ.get("SKEIN_ATTN_DECODE", _DECODE_DEFAULT)
+    if kernel in ("tc", "auto"):
+        kernel = "mma"
+    if kv_cache.shape[3] % 16 != 0 or Hq // Hkv > 16:
+        kernel = "scalar"
+    split_tokens = 0
+    if splits is None and kernel == "scalar":
+        splits = _scalar_splits(B, Hkv, ctx_hint, ws.sm_count)
+    elif splits is None:
+        splits, split_tokens = split_plan(B, Hkv, ctx_hint, ws.sm_count, Hq // Hkv)
     wsf, ctr = (None, None)
     if splits > 1:
         scratch = ws.attn_scratch(B, Hq, Hkv, splits)
@@ -552,16 +575,13 @@ def attn_decode(q, kv_cache, block_table, seq_lens, Hq, Hkv, D, scale=None, out=
             _lib.check(rc, "attn_decode_tc")
             _lib.count_launch()
             return out
-    impl = impl or os.environ.get("SKEIN_ATTN_DECODE", _DECODE_DEFAULT)
-    if impl in ("tc", "auto"):
-        impl = "mma"
-    if kv_cache.shape[3] % 16 != 0 or Hq // Hkv > 16:
-        impl = "scalar"
-    fn = _lib.lib().skein_attn_decode_mma if impl == "mma" else _lib.lib().skein_attn_decode
-    rc = fn(
-        q.data_ptr(), q.stride(0), kv_cache.data_ptr(), block_table.data_ptr(), seq_lens.data_ptr(), out.data_ptr(),
-        _lib.ptr(wsf), _lib.ptr(ctr), ws.status.data_ptr(), B, Hq, Hkv, D, kv_cache.shape[3], block_table.stride(0),
-        kv_cache.shape[0], splits, float(scale), _lib.stream_ptr())
+    args = (q.data_ptr(), q.stride(0), kv_cache.data_ptr(), block_table.data_ptr(), seq_lens.data_ptr(), out.data_ptr(),
+            _lib.ptr(wsf), _lib.ptr(ctr), ws.status.data_ptr(), B, Hq, Hkv, D, kv_cache.shape[3], block_table.stride(0),
+            kv_cache.shape[0], splits)
+    if kernel == "mma":
+        rc = _lib.lib().skein_attn_decode_mma(*args, split_tokens, float(scale), _lib.stream_ptr())
+    else:
+        rc = _lib.lib().skein_attn_decode(*args, float(scale), _lib.stream_ptr())
     _lib.check(rc, "attn_decode")
     _lib.count_launch()
     return out
@@ -585,8 +605,9 @@ def attn_decode_rope(qkv, positions, block_table, cos_sin, kv_cache, seq_lens, H
     if out is None:
         out = torch.empty(B, Hq * D, dtype=torch.bfloat16, device=qkv.device)
     ws = workspace()
+    split_tokens = 0
     if splits is None:
-        splits = pick_splits(B, Hkv, ctx_hint, ws.sm_count, Hq // Hkv)
+        splits, split_tokens = split_plan(B, Hkv, ctx_hint, ws.sm_count, Hq // Hkv)
     wsf, ctr = (None, None)
     if splits > 1:
         scratch = ws.attn_scratch(B, Hq, Hkv, splits)
@@ -607,7 +628,7 @@ def attn_decode_rope(qkv, positions, block_table, cos_sin, kv_cache, seq_lens, H
         qkv.data_ptr(), qkv.stride(0), kv_cache.data_ptr(), block_table.data_ptr(), seq_lens.data_ptr(),
         positions.data_ptr(), cos_sin.data_ptr(), cos_sin.shape[0], out.data_ptr(), _lib.ptr(wsf), _lib.ptr(ctr),
         ws.status.data_ptr(), B, Hq, Hkv, D, kv_cache.shape[3], block_table.stride(0), kv_cache.shape[0], splits,
-        float(scale), _lib.stream_ptr())
+        split_tokens, float(scale), _lib.stream_ptr())
     _lib.check(rc, "attn_decode_rope")
     _lib.count_launch()
     return out

@@ -174,12 +174,12 @@ def window_attn(q, spec, inp, cache, page_size, out, out_scale=1.0, mix: HeadMix
             page_size, bt.stride(0), cache.shape[0], C.byref(r), _lib.stream_ptr())
     else:
         B, reach = q.shape[0], spec.window + spec.keep_first if spec.window else spec.chunk or inp.ctx_hint
-        splits = F.pick_splits(B, K, min(inp.ctx_hint, reach), ws.sm_count, H * spec.maps // K)
+        splits, tokens = F.split_plan(B, K, min(inp.ctx_hint, reach), ws.sm_count, H * spec.maps // K)
         scratch = ws.attn_scratch(B, H * spec.maps, K, splits) if splits > 1 else None
         splits, (wsf, ctr) = (splits, scratch) if scratch is not None else (1, (None, None))
         rc = _lib.lib().skein_attn_decode_window(
             q.data_ptr(), q.stride(0), cache.data_ptr(), bt.data_ptr(), inp.seq_lens.data_ptr(), out.data_ptr(), out.stride(0), _lib.ptr(wsf),
-            _lib.ptr(ctr), ws.status.data_ptr(), B, H, K, KW, page_size, bt.stride(0), cache.shape[0], splits, C.byref(r), _lib.stream_ptr())
+            _lib.ptr(ctr), ws.status.data_ptr(), B, H, K, KW, page_size, bt.stride(0), cache.shape[0], splits, tokens, C.byref(r), _lib.stream_ptr())
     _lib.check(rc, "window_attn")
     _lib.count_launch()
     return out
