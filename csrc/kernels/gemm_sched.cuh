@@ -127,11 +127,13 @@ __device__ __forceinline__ void build_sched(Sched& sched, const SkeinGemmParams&
     const int by_k = sched.KB / 4 > 0 ? sched.KB / 4 : 1;   // at least 4 K-blocks per piece
     if (sp > by_k) sp = by_k;
     if (k_elems_per_block == 128) {
-      // e4m3 weights: a K-block costs a CTA its conversion whatever the memory does, so the longest piece decides and an idle CTA is lost.
-      // Aligned pieces while they are at most 6 K-blocks longer than an equal share, which is what its second partial tile costs:
-      // 10240 x 8192 (80 tiles of 64, whole) 38.9 against 32.8 us, 8192 x 28672 (64 of 224 in two) 67.6 / 62.8, 8192 x 8192 27.1 / 27.7,
-      // gate/up 3584 x 8192 (28 of 64 in five) 23.6 / 27.1
-      if ((sched.KB + sp - 1) / sp <= (int)((sched.TK + grid - 1) / grid) + 6) sched.split = sp;
+      // e4m3 weights: a K-block costs a CTA its conversion whatever the memory does, so the longest piece decides, and an equal share pays with
+      // a second partial tile. Aligned pieces up to 12 K-blocks longer than an equal share win by what the partials cost (7168 x 8192 at 16 tokens
+      // 24.2 against 24.9 us, 6144 x 4096 at 256 28.9 / 40.8, gate/up 8192 x 8192 at 100 58.2 / 79.2); whole tiles, which have no partials, up to
+      // 40 longer where those are large (7168 x 8192 at 256 tokens 45.9 / 56.6, gate/up 3584 x 18944 at 256 107 / 124, but gate/up 10240 x 8192 at 32
+      // 52.7 / 49.0). Beyond, equal shares: 8192 x 28672 (64 tiles of 224 in two) at 100 tokens 76.6 / 72.9.
+      const int longer = (sched.KB + sp - 1) / sp - (int)((sched.TK + grid - 1) / grid), cols = p.n_tile * (p.mode == 1 ? 2 : 1);
+      if (longer <= 12 || (sp == 1 && longer <= 40 && cols >= 112)) sched.split = sp;
       return;
     }
     // with fewer than two CTAs per tile, whole tiles on `acc` CTAs beat the line cut while the longer

@@ -35,3 +35,12 @@ def test_rings(features, K, rows, tile, unit):
         total, off = s * u, (1.1 * ea + 2.0 ** -20 * s.abs()) * (u.abs() + eu) + (s.abs() + 1.1 * ea) * eu
     assert bool(((y.double() - total).abs() <= off + 2.0 ** -8 * (total.abs() + off)).all())
     assert torch.equal(y, fp8.linear_a16(x, q, swiglu=unit, n_tile=tile))
+
+
+# either side of the lines at which a tile is cut into aligned pieces, taken whole or dealt as equal shares (csrc/kernels/gemm_sched.cuh), features x K at `rows`
+# tokens: pieces 7 and 15 K-blocks longer than an equal share, whole tiles 8, 15 and 29 longer, with a small token tile and a large one
+@pytest.mark.parametrize("features,K,rows,tile,unit", [(7168, 8192, 16, 16, False), (8192, 28672, 16, 16, False), (8192, 8192, 200, 128, False),
+                                                       (7168, 8192, 200, 128, False), (10240, 8192, 16, 16, False), (10240, 8192, 100, 112, False),
+                                                       (3584, 8192, 200, 64, True), (10240, 8192, 32, 32, True), (3584, 18944, 160, 64, True)])
+def test_cuts(features, K, rows, tile, unit):
+    test_rings(features, K, rows, tile, unit)
