@@ -101,3 +101,24 @@ def test_repeats_are_bitwise_alike(monkeypatch):
     _pair_only(monkeypatch)
     x, w = _inputs(300, 2048, 4096)
     assert torch.equal(ops.linear(x, w), ops.linear(x, w))
+
+
+@pytest.mark.parametrize("rows,features,K", [(300, 2048, 2048), (2304, 2304, 256), (257, 1000, 1032)])       # cut tiles; whole ones; features inside a CTA's rows
+def test_residuals_in_place_and_rows_of_any_pitch(monkeypatch, rows, features, K):
+    _pair_only(monkeypatch)
+    x, w = _inputs(rows, features, K)
+    want, bound = _sum(x, w)
+    half = torch.randn(rows, features, device=DEV).bfloat16()
+    total = half.clone()
+    ops.linear(x, w, out=total, residual=total)
+    _close(total, want + half.double(), bound)
+    for pitch, first in ((8, 4), (3, 1), (2, 2)):                                # whole 16-byte groups; single values; pairs, that are no groups of four
+        for dtype in (torch.float32, torch.bfloat16):
+            wide = torch.randn(rows, features + pitch, device=DEV).to(dtype)
+            before, cols = wide.clone(), slice(first, first + features)
+            ops.linear(x, w, out=wide[:, cols], residual=wide[:, cols], out_f32=dtype == torch.float32, relu2_cols=features // 2 + 3)
+            sq = want.clone()
+            sq[:, :features // 2 + 3] = sq[:, :features // 2 + 3].clamp(min=0).square()
+            _close(wide[:, cols], sq + before[:, cols].double(), (2 * want.abs() + bound + 1) * bound, bf16=dtype == torch.bfloat16)
+            wide[:, cols] = before[:, cols]
+            assert torch.equal(wide, before)
