@@ -45,6 +45,7 @@ struct PairSched {
   int pre[SKEIN_MAX_GROUPS + 1], cnt[SKEIN_MAX_GROUPS], off[SKEIN_MAX_GROUPS], ntile[SKEIN_MAX_GROUPS], cols[SKEIN_MAX_GROUPS];
   int MT, KB, U;
   int R, split;      // the first R tiles are cut into `split` pieces along K: piece i of tile u is pair i * R + u's
+  int halves;        // whole tiles are summed in two halves of K (see pair_sched)
 };
 
 // number of tiles of a group of c rows, and tokens per tile
@@ -85,11 +86,16 @@ __device__ __forceinline__ void pair_sched(PairSched& s, const SkeinGemmParams& 
   s.pre[p.G] = s.U = (int)acc;
   s.split = pair_split(s.U % pairs, s.KB, pairs);
   s.R = s.split > 1 ? s.U % pairs : 0;
+  // Outputs kept in 32 bits: the tensor core's sums lose with the length of the chain, and one accumulator over all of K was further off 64 bits than the
+  // pieces that the streaming kernel cuts (K of 22528: 2.6e-5 of the norm against 1.9e-5, 4096: 4.4e-6 / 3.9e-6). Each half of K has an accumulator of
+  // its own, added at the end; the next tile then waits for the epilogue. Outputs in bf16 round away 1.7e-3.
+  s.halves = p.mode == 0 && p.out_f32 && s.KB >= 32;
 }
 
 // A pair's work: its piece of a cut tile, then whole tiles R + c, R + c + pairs, ...
 struct PairWalk {
   int piece, next;
+  bool cut = false, more = false;      // of the step just taken: a piece of a cut tile; a first half, whose second one comes next
   __device__ __forceinline__ PairWalk(const PairSched& s, int c) : piece(c < s.R * s.split ? c : -1), next(s.R + c) {}
   __device__ __forceinline__ bool step(const PairSched& s, int pairs, int& u, int& kb0, int& kb1) {
     if (piece >= 0) {
@@ -99,11 +105,16 @@ struct PairWalk {
       kb0 = i * s.KB / s.split;
       kb1 = (i + 1) * s.KB / s.split;
       piece = -1;
+      cut = true;
       return true;
     }
+    cut = false;
     if (next >= s.U) return false;
-    u = next; kb0 = 0; kb1 = s.KB;
-    next += pairs;
+    u = next;
+    more = s.halves && !more;      // (false before the first step)
+    kb0 = s.halves && !more ? s.KB / 2 : 0;
+    kb1 = more ? s.KB / 2 : s.KB;
+    if (!more) next += pairs;
     return true;
   }
 };
@@ -412,7 +423,6 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
     uint32_t seg = 0;
     int u, kb0, kb1, buf = 0;
     for (; ok && walk.step(sched, pairs, u, kb0, kb1); ++seg) {
-      const bool whole = kb0 == 0 && kb1 == KB;
       if (parked >= 0) {
         reduce_parked();
         if (!ok) break;
@@ -426,11 +436,13 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
         break;
       }
       tc_fence_after();
-      const uint32_t t_acc = tmem_base + b * PAIR_COLS + ((uint32_t)(q * 32) << 16);
+      if (walk.more) continue;               // the first half stays in its accumulator until the second one is there
+      const bool halves = sched.halves && !walk.cut;
+      const uint32_t t_acc = tmem_base + b * PAIR_COLS + ((uint32_t)(q * 32) << 16), t_first = tmem_base + (b ^ 1) * PAIR_COLS + ((uint32_t)(q * 32) << 16);
       const int cols = sched.cols[un.g];
       const int valid = min(cols, sched.cnt[un.g] - un.n * cols);
       const long long row0 = (long long)sched.off[un.g] + (long long)un.n * cols;
-      if (!whole) {
+      if (walk.cut) {
         float* ws = p.workspace + (size_t)blockIdx.x * slot_elems;
         for (int c0 = 0; c0 < valid; c0 += 32) {
           uint32_t v[32];
@@ -488,12 +500,15 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
 #pragma unroll
               for (int j = 0; j < 32; ++j) rv[j] = __ldcg(res + (size_t)min(c0 + j, valid - 1) * p.ldo);
             }
+            uint32_t v1[32];
+            if (halves) tmem_ld32(t_first + c0, v1);
             tmem_ld_wait();
             if (f < p.F) {
               float* out = (float*)p.out + first;
 #pragma unroll
               for (int j = 0; j < 32; ++j) {
                 float y = __uint_as_float(v[j]);
+                if (halves) y += __uint_as_float(v1[j]);
                 if (f < p.relu2_cols) y = relu2(y);
                 if (p.residual != nullptr) y += rv[j];
                 if (c0 + j < valid) out[(size_t)(c0 + j) * p.ldo] = y;
@@ -527,7 +542,10 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
       }
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive_cluster(leader_tempty[b]);
+      if (lane == 0) {
+        if (halves) mbar_arrive_cluster(leader_tempty[b ^ 1]);
+        mbar_arrive_cluster(leader_tempty[b]);
+      }
     }
     if (ok && parked >= 0) reduce_parked();
   }

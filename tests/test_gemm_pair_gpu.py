@@ -122,3 +122,20 @@ def test_residuals_in_place_and_rows_of_any_pitch(monkeypatch, rows, features, K
             _close(wide[:, cols], sq + before[:, cols].double(), (2 * want.abs() + bound + 1) * bound, bf16=dtype == torch.bfloat16)
             wide[:, cols] = before[:, cols]
             assert torch.equal(wide, before)
+
+
+@pytest.mark.parametrize("rows,features,K", [(1000, 2304, 4096), (2100, 2304, 14336), (1000, 4096, 22528), (300, 512, 2048)])
+def test_sums_in_32_bits_are_as_good_as_the_streaming_kernels(monkeypatch, rows, features, K):
+    """The tensor core's fp32 sums lose with the length of the chain: outputs kept in 32 bits must not be further off than the kernel that cuts K."""
+    x, w = _inputs(rows, features, K)
+    want = _sum(x, w)[0]
+    monkeypatch.setattr(F, "pair_gemm_ok", lambda p, rows: False)
+    off = (ops.linear(x, w, out_f32=True).double() - want).norm()
+    _pair_only(monkeypatch)
+    y = ops.linear(x, w, out_f32=True)
+    res = torch.randn(rows, features, device=DEV)
+    total = ops.linear(x, w, out=res.clone(), residual=res, out_f32=True)
+    torch.cuda.synchronize()
+    ops.workspace().check_status()
+    assert (y.double() - want).norm() <= 1.02 * off
+    assert torch.equal(total, y + res) and torch.equal(y, ops.linear(x, w, out_f32=True))
