@@ -6,7 +6,7 @@
 // 16 + 16 mma.sync m16n8k16 instead of ~4k scalar FMAs per warp, and K/V tiles stream from the
 // cache into shared memory with cp.async while earlier tiles are being multiplied.
 //
-//   grid = (Hkv, B, splits), 128 threads. The split's range of 16-token tiles is dealt round-robin
+//   grid = (splits, Hkv, B) or (Hkv, B, splits), 128 threads. The split's range of 16-token tiles is dealt round-robin
 //   to the 4 warps. Each warp runs its own 3- or 6-stage pipeline (no CTA-wide barrier in the loop):
 //       cp.async tile i+2 (K 4 KB + V 4 KB, XOR-swizzled rows)      wait tile i
 //       S = Q K^T  (2 n-tiles x 8 k-steps)   online softmax in registers   O += P V (16 n-tiles)
@@ -58,6 +58,7 @@ struct AttnMmaParams {
   int* status;
   long long q_stride;
   int B, Hq, Hkv, G, page_size, max_blocks, num_pages, splits;   // Hq, G: query rows, the maps of differential heads counted apart
+  int split_last;                                                 // the grid is (Hkv, B, splits) instead of (splits, Hkv, B)
   int split_log2;                                                 // log2 of the tokens that make a split worth its merge (0: every split is used)
   float scale_log2e, cap_in, cap_log2e;      // (cap_log2e 0: scores are not capped; attn_cap)
   // optional fusion of RoPE and the KV append of the new token (cos_sin == nullptr: q is already rotated and
@@ -105,10 +106,10 @@ __global__ void __launch_bounds__(AM_THREADS) attn_decode_mma_kernel(const AttnM
   constexpr int AM_WARP_BYTES = AM_STAGES * AM_STAGE_BYTES;
   constexpr int CH = AM_D / 8, KS = AM_D / 16, ND = AM_D / 8;    // 16-byte chunks of a row, k-steps of Q K^T, n-tiles of P V
   extern __shared__ __align__(128) uint8_t am_smem[];
-  __shared__ int is_last;
+  __shared__ int is_last, splits_used;      // (kept here: a register more over the tile loop made it 6 % slower)
   pdl_trigger();
   pdl_wait();   // q, the cache and the sequence lengths come from earlier kernels of the step
-  const int split = blockIdx.z, kvh = blockIdx.x, b = blockIdx.y;
+  const int split = p.split_last ? blockIdx.z : blockIdx.x, kvh = p.split_last ? blockIdx.x : blockIdx.y, b = p.split_last ? blockIdx.y : blockIdx.z;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int G = p.G, ps = p.page_size;
   const int len = p.seq_lens[b];
@@ -119,8 +120,8 @@ __global__ void __launch_bounds__(AM_THREADS) attn_decode_mma_kernel(const AttnM
   const int keep = p.r.keep_first, tile_lo = lo / AM_TILE, unit = p.r.window > 0 || p.r.chunk > 0 ? AM_TILE : ps;
   const int kept = min((keep + AM_TILE - 1) / AM_TILE, tile_lo), hop = tile_lo - kept;     // tiles of the first tokens; skipped behind them
   const int row_len = len - hop * AM_TILE;
-  const int ns = p.split_log2 > 0 ? max(1, min(p.splits, (row_len + (1 << (p.split_log2 - 1))) >> p.split_log2)) : p.splits;
-  int per = (row_len + ns - 1) / ns;
+  const int used = p.split_log2 > 0 ? max(1, min(p.splits, (row_len + (1 << (p.split_log2 - 1))) >> p.split_log2)) : p.splits;
+  int per = (row_len + used - 1) / used;
   per = (per + unit - 1) / unit * unit;
   const int t_begin = split * per, t_end = min(t_begin + per, row_len);
   const int tile_begin = t_begin / AM_TILE;
@@ -173,7 +174,7 @@ __global__ void __launch_bounds__(AM_THREADS) attn_decode_mma_kernel(const AttnM
     // the barrier below orders these stores before the asynchronous copies that read them back
     if (pos >= 0) {
       int s_app = per > 0 ? pos / per : 0;
-      if (s_app > ns - 1) s_app = ns - 1;
+      if (s_app > used - 1) s_app = used - 1;
       if (s_app == split) {
         int pg = p.block_table[(size_t)b * p.max_blocks + pos / ps];
         if (pg < 0 || pg >= p.num_pages) {
@@ -196,7 +197,8 @@ __global__ void __launch_bounds__(AM_THREADS) attn_decode_mma_kernel(const AttnM
       }
     }
   }
-  if (split >= ns) return;      // (here, so that the queries' loads do not wait for the length's)
+  if (split >= used) return;      // (here, so that the queries' loads do not wait for the length's)
+  if (tid == 0) splits_used = used;
   __syncthreads();
   uint32_t qf[KS][4];
 #pragma unroll
@@ -392,6 +394,7 @@ __global__ void __launch_bounds__(AM_THREADS) attn_decode_mma_kernel(const AttnM
       O_g[g] = O; M_g[g] = M; L_g[g] = L;
     }
   }
+  const int ns = splits_used;
   if (ns == 1) {
     if (AM_D == AM_THREADS && p.r.maps == 2) {
       store_pairs([&](int g) { return O_g[g] * attn_norm(M_g[g], L_g[g], sink_of(g)); });
@@ -470,10 +473,14 @@ static int attn_decode_mma_go(AttnMmaParams& p, float* ws, void* stream) {
   }
   p.ws_o = ws;
   p.ws_ml = ws ? ws + (size_t)p.B * p.Hq * p.splits * AM_D : nullptr;
-  const dim3 grid(p.Hkv, p.B, p.splits);      // (splits last: those that leave at once must not take half of the SMs from the others)
   int sms = 0;
   if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0) sms = 148;
-  if ((long long)p.splits * p.Hkv * p.B <= sms)
+  // A sequence's splits side by side, which end and are merged together (16 splits of 8 heads: 24.9 us, 26.8 with the splits last). With more CTAs
+  // than SMs the splits come last: those that leave at once would take every other place from those that work (16 sequences of 2000 tokens x 8 heads
+  // under a hint of 8192: 37 us, 41 side by side).
+  p.split_last = (long long)p.splits * p.Hkv * p.B > sms;
+  const dim3 grid = p.split_last ? dim3(p.Hkv, p.B, p.splits) : dim3(p.splits, p.Hkv, p.B);
+  if (!p.split_last)
     return (int)launch_pdl(attn_decode_mma_kernel<6, AM_D>, grid, dim3(AM_THREADS), (size_t)am_smem_bytes(6, AM_D), (cudaStream_t)stream, p);
   return (int)launch_pdl(attn_decode_mma_kernel<3, AM_D>, grid, dim3(AM_THREADS), (size_t)am_smem_bytes(3, AM_D), (cudaStream_t)stream, p);
 }

@@ -497,13 +497,17 @@ def split_plan(B, Hkv, ctx_hint, sm_count=148, group=16):
     for the others to end (32 pairs of 8000 tokens: 38.5 us with 8, 51.8 with 10; 160 pairs of 2048: 44 whole, 60 in two). A split adds a workspace
     round trip and a merge, so that it needs more tokens the more pairs there are: with 113 to 148 pairs two splits cost 2 to 7 % for
     sequences of one length below 8000 tokens. Against one CTA per SM and 512 tokens per split, us, one length / lengths from a fifth up:
-    40 pairs of 8000 47.7 / 42.3 -> 45.2 / 33.0, of 1024 17.3 / 16.2 -> 16.8 / 14.7; 80 of 4096 58.7 / 55.5 -> 45.1 / 36.7; 8 of 768 16.8 -> 14.0.
-    group: query heads per kv head, for the scratch that the partials share (Workspace.attn_scratch)."""
+    40 pairs of 8000 47.7 / 42.3 -> 45.2 / 33.0, of 1024 17.3 / 16.2 -> 16.8 / 14.7; 80 of 4096 58.7 / 55.5 -> 45.1 / 36.7; 8 of 768 16.8 -> 13.5.
+    group: query heads per kv head: a merge takes longer the more there are (24 pairs of 8 heads, 700 tokens: 16.3 whole, 17.1 in three), and
+    their partials share the scratch (Workspace.attn_scratch)."""
     if os.environ.get("SKEIN_ATTN_SPLITS"):
         return int(os.environ["SKEIN_ATTN_SPLITS"]), 0
     pairs = max(B * Hkv, 1)
     one = sm_count // pairs
-    tokens = 256 if pairs <= 40 and ctx_hint >= 768 else 512 if pairs <= 80 else 1000 if pairs <= 112 else 4000
+    if pairs <= 40 and ctx_hint >= (768 if group < 8 else 1024):
+        tokens = 128 if pairs <= 16 else 256
+    else:
+        tokens = 512 if pairs <= 80 else 1000 if pairs <= 112 else 4000
     fit = one if one >= 6 else 2 * sm_count // pairs
     return max(1, min(fit, ctx_hint // tokens, sm_count * Workspace.MAX_GROUP // (pairs * group), 16)), 1 << round(math.log2(tokens))
 

@@ -19,7 +19,7 @@ def test_rule():
                 splits, tokens = F.split_plan(B, Hkv, ctx, 148, group)
                 pairs = B * Hkv
                 assert 1 <= splits <= 16 and (splits == 1 or pairs * splits <= 2 * 148) and pairs * group * splits <= max(148 * 16, pairs * group)
-                assert tokens >= 256 and (splits == 1 or ctx >= splits * 256)
+                assert tokens >= 128 and (splits == 1 or ctx >= splits * 128)
     assert F.split_plan(5, 8, 8000, 148, 4)[0] == 7 and F.split_plan(1, 8, 4096, 148, 4)[0] == 16 and F.split_plan(20, 8, 8000, 148, 4)[0] == 1
 
 
