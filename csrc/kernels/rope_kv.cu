@@ -144,13 +144,18 @@ extern "C" int skein_rope_kv_append(void* qkv, const int* positions, const int* 
                                     int Hkv, int D, int max_pos, int num_pages, int* status, void* stream) {
   if (T == 0) return 0;
   if (D % 2 != 0 || D / 2 > 1024) return -1;
-  if (D % 16 == 0 && D <= 2048 && (((uintptr_t)qkv | (uintptr_t)kv_cache | (uintptr_t)cos_sin) & 15) == 0) {
+  // A CTA per token walks the heads one after the other: it takes enough tokens to fill the GPU with them, and heads to fill its threads. CTA per
+  // token and head / CTA per token, us: 48 heads of 128 2.7 / 4.4 for one token, 5.3 / 5.8 for 128, 8.5 / 6.5 for 256; 80 heads 4.8 / 6.9 for 64, 7.6 / 7.5
+  // for 128; 12 heads of 64 3.7 / 4.4 for 256, 8.2 / 4.6 for 1000; 3 heads of 128 8.5 / 9.3 for 4096.
+  const int heads = Hq + 2 * Hkv;
+  if (D % 16 == 0 && D <= 2048 && (long long)T * heads >= 9000 && heads * (D / 16) >= 32 &&
+      (((uintptr_t)qkv | (uintptr_t)kv_cache | (uintptr_t)cos_sin) & 15) == 0) {
     skein::rope_kv_append_vec_kernel<<<T, 128, 0, (cudaStream_t)stream>>>(
         (__nv_bfloat16*)qkv, positions, seq_of_token, block_table, max_blocks, cos_sin, (__nv_bfloat16*)kv_cache,
         page_size, Hq, Hkv, D, max_pos, num_pages, status);
     return (int)cudaGetLastError();
   }
-  dim3 grid(T, Hq + 2 * Hkv);
+  dim3 grid(T, heads);
   skein::rope_kv_append_kernel<<<grid, D / 2, 0, (cudaStream_t)stream>>>(
       (__nv_bfloat16*)qkv, positions, seq_of_token, block_table, max_blocks, cos_sin, (__nv_bfloat16*)kv_cache,
       page_size, Hq, Hkv, D, max_pos, num_pages, status);

@@ -87,3 +87,30 @@ def test_route(T, H, E, k):
         again = ops.router_plan(ids, E, first, count)
         _done()
         assert torch.equal(again[0], want[0]) and torch.equal(again[2].view(-1), want[2].view(-1))
+
+
+# both sides of the line between a CTA per token and head and one per token: enough tokens, head sizes whose pairs do not divide the threads, heads that leave
+# threads idle, more heads than fit at once, no 16-byte halves
+@pytest.mark.parametrize("T,D,Hq,Hkv", [(1285, 128, 5, 1), (1286, 128, 5, 1), (2250, 64, 2, 1), (1500, 48, 4, 1), (260, 16, 33, 1), (300, 128, 28, 4), (9000, 16, 2, 1),
+                                        (1300, 24, 5, 1), (190, 64, 40, 4)])
+def test_rope_of_many_tokens(T, D, Hq, Hkv):
+    g, page, S = _gen(), 16, 3
+    per = (T + S - 1) // S
+    qkv = torch.randn(T, (Hq + 2 * Hkv) * D, device=DEV, generator=g).bfloat16()
+    at = torch.arange(T, device=DEV)
+    pos, seq = (at % per).int(), (at // per).int()
+    pos[7] = -1
+    nb = (per + page - 1) // page
+    table = torch.randperm(S * nb, device=DEV, generator=g).int().view(S, nb)
+    cs = torch.randn(per, D // 2, 2, device=DEV, generator=g)
+    cache = torch.zeros(S * nb, 2, Hkv, page, D, dtype=torch.bfloat16, device=DEV)
+    live = pos >= 0
+    q2, c2 = qkv[live].cpu(), cache.clone().cpu()
+    ref.rope_kv_append(q2, pos[live].cpu(), seq[live].cpu(), table.cpu(), cs.cpu(), c2, Hq, Hkv, D)
+    before = qkv.clone()
+    ops.rope_kv_append(qkv, pos, seq, table, cs, cache, Hq, Hkv, D)
+    _done()
+    for a, b in ((qkv[live][:, :Hq * D].cpu(), q2[:, :Hq * D]), (cache.cpu(), c2)):
+        # x c - y s in fp32, rounded to bf16 (2^-8 of it) here and there; what cancels is bounded by the two products
+        assert bool(((a.float() - b.float()).abs() <= 2.0 ** -7 * b.float().abs() + 2.0 ** -20).all())
+    assert torch.equal(qkv[~live], before[~live]) and torch.equal(qkv[:, Hq * D:], before[:, Hq * D:])
