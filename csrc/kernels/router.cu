@@ -351,8 +351,9 @@ extern "C" int skein_router_topk(const void* x, const void* wg, int T, int H, in
   if (E > RT_MAX_E || topk > RT_MAX_K || topk > E || H % 8 != 0) return -1;
   const RouterOut o{expert_ids, expert_w, logits_out, counts, offsets, row_of, src_token, e_first, e_count, done_counter};
   const __nv_bfloat16 *xb = (const __nv_bfloat16*)x, *wb = (const __nv_bfloat16*)wg;
-  // (11 us either way at 200 tokens x 4096 and 8 experts; 14 against 10 at 296)
-  if (T >= 256 && H % 32 == 0) router_rows_kernel<<<(T + RR_TOKENS - 1) / RR_TOKENS, 512, 0, (cudaStream_t)stream>>>(xb, wb, T, H, E, topk, o);
+  // Few tokens are few tiles, and up to four experts leave half of a tile empty. CTA per token / tiles, us: 8 experts x 4096 15.5 / 13.1 at 256 tokens,
+  // x 8192 19.4 / 17.6; 4 experts x 1024 8.5 / 7.9, x 8192 12.1 / 15.1, at 300 13.4 / 15.5, at 512 19.7 / 16.1.
+  if (T >= 256 && H % 32 == 0 && (E > 4 || H <= 2048 || T >= 512)) router_rows_kernel<<<(T + RR_TOKENS - 1) / RR_TOKENS, 512, 0, (cudaStream_t)stream>>>(xb, wb, T, H, E, topk, o);
   else router_topk_kernel<<<T, 512, 0, (cudaStream_t)stream>>>(xb, wb, T, H, E, topk, o);
   return (int)cudaGetLastError();
 }

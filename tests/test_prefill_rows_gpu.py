@@ -114,3 +114,9 @@ def test_rope_of_many_tokens(T, D, Hq, Hkv):
         # x c - y s in fp32, rounded to bf16 (2^-8 of it) here and there; what cancels is bounded by the two products
         assert bool(((a.float() - b.float()).abs() <= 2.0 ** -7 * b.float().abs() + 2.0 ** -20).all())
     assert torch.equal(qkv[~live], before[~live]) and torch.equal(qkv[:, Hq * D:], before[:, Hq * D:])
+
+
+# up to four experts: rows of 2048 and less take the tiles from 256 tokens on, longer ones from 512
+@pytest.mark.parametrize("T,H,E,k", [(255, 2048, 4, 1), (256, 2048, 4, 2), (300, 4096, 4, 1), (511, 2080, 3, 2), (512, 2080, 3, 2), (520, 8192, 4, 1)])
+def test_route_of_few_experts(T, H, E, k):
+    test_route(T, H, E, k)
