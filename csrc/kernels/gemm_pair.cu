@@ -591,7 +591,7 @@ static int pair_grid() {
 
 // Tokens of a tile for `rows` rows: the width for which the rounds of whole and cut tiles cost least, where a K-block of a tile costs the
 // bytes that it stages (128 weight rows and half of its tokens per CTA). Narrower than 256 pays where that fills a round: 512 rows of 6144
-// features are 72 tiles of 192 instead of 48 of 256 (see the sizes at PAIR_MIN_ROWS in ops/functional.py).
+// features are 72 tiles of 192 instead of 48 of 256 (see the sizes at pair_gemm_ok in ops/functional.py).
 static int pair_cap(int rows, int MT, int KB, int pairs) {
   long long best = 0;
   int cap = PAIR_COLS;

@@ -114,17 +114,38 @@ def pick_n_tile(rows_hint: int, dual: bool, features: int = 0) -> int:
     return max(16, min(cap, _round_up(max(rows_hint, 1), 16)))
 
 
-PAIR_MIN_ROWS = 96        # of a group
-
-
 def pair_gemm_ok(p: "_lib.GemmParams", rows: int) -> bool:
     """Whether a product with `rows` rows in each of its groups runs on pairs of CTAs (csrc/kernels/gemm_pair.cu) instead of the streaming
-    kernel. Below that the weights' bytes decide and the streaming kernel, which spreads them over all SMs whatever the number of tiles, is
-    as quick or quicker; one group without a gate/up pair has few tiles, so that it changes sides later. Measured, streaming / pairs, us:
-    gate/up 14336 x 4096 53 / 56 at 64 rows, 60 / 58 at 96, 67 / 57 at 128, 150 / 89 at 512, 1080 / 608 at 4096; eight experts of it 296 / 285 at 64 rows
-    each, 312 / 294 at 96, 540 / 336 at 192; 10240 x 8192 57 / 61 at 128 rows, 67 / 65 at 192, 94 / 66 at 512, 673 / 444 at 4096."""
-    many = p.G > 1 or p.mode == 1
-    return rows >= (PAIR_MIN_ROWS if many else 2 * PAIR_MIN_ROWS) and p.F >= 256 and p.K >= 256
+    kernel. The pairs' 256 x 256 tiles pay where the products bound the time: many rows, long rows of weights, enough tiles. Else the streaming kernel
+    is as quick or quicker: it spreads the weights' bytes over all SMs whatever the number of tiles, and has narrower tiles where few of them
+    leave SMs idle. Measured over features x K x rows, streaming / pairs, us:
+
+    gate/up, one group: 14336 x 4096 57 / 60 at 96 rows, 61 / 62 at 128, 173 / 92 at 512, 1104 / 1042 at 4096; 2048 x 2048 17 / 15 at 96.
+    gate/up, groups: 8 x 14336 x 4096 331 / 332 at 96 rows each, 493 / 350 at 128 (uneven), 1187 / 893 at 512; 64 x 512 x 1024 59 / 64 at 128, 97 / 75 at
+        192; 2 x 1024 x 1024 17 / 22 at 256.
+    groups: 8 x 4096 x 14336 187 / 179 at 128, 573 / 378 at 512; 64 x 1408 x 2048 103 / 101 at 128; 8 x 2048 x 2048 26 / 30 at 256, 54 / 38 at 400; 64 x 512 x
+        1024 61 / 73 at 512; 2 x 4096 x 4096 36 / 38 at 512, 82 / 56 at 1024.
+    one group, up to 256 rows: 1024 x 1024 15 / 11 at 192, 4096 x 4096 21 / 22, 8192 x 8192 41 / 46, 4096 x 14336 36 / 40.
+    one group, more rows: 4096 x 4096 42 / 28 at 512, 136 / 88 at 4096; 6144 x 4096 28 / 32 at 512, 70 / 45 at 1000; 4096 x 14336 96 / 49 at 320; 4608 x 3584
+        31 / 33 at 1000, 132 / 85 at 4096; 4096 x 2048 33 / 36 at 2048, 66 / 44 at 3000; 2048 x 2048 15 / 19 at 512; 8192 x 512 51 / 69 at 4096.
+    the same with a bf16 residual: 1024 x 1024 24 / 14 at 320, 4096 x 4096 267 / 61 at 2048.
+    the same in 32 bits, where a tile's sums in two halves of K leave the epilogue in the open: 4096 x 22528 234 / 142 at 1000; 4096 x 4096 80 / 46 at
+        1000, 70 / 84 at 2048; 2048 x 2048 23 / 25 at 1000."""
+    F, K, G = p.F, p.K, p.G
+    if F < 256 or K < 256:
+        return False
+    if p.mode == 1 and G == 1:
+        return rows >= (96 if F * K <= 1 << 23 else 128)
+    if p.mode == 1:
+        return rows >= (192 if G >= 32 and F * K < 1 << 20 else 128) and (G >= 8 or F * K >= 1 << 21)
+    if G > 1:
+        return K >= 1280 and (rows >= 128 and (G * F >= 1 << 16 or K >= 8192) or rows >= 384 and K >= 2048 and G * rows * F >= 5 << 20)
+    if rows <= 256:
+        return rows >= 192 and F * K <= 1 << 23
+    out = rows * F
+    if p.out_f32:
+        return out >= 1 << 20 and (K >= 8192 or K >= 4096 and out < 1 << 23)
+    return bool(p.residual) or K >= 4096 and out >= 15 << 18 or K >= 2048 and out >= 9 << 20 or K >= 8192 and out >= 1 << 20
 
 
 def _gemm_launch(p: "_lib.GemmParams", what: str, cfg: dict | None = None, rows: int = 0):
