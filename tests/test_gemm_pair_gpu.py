@@ -139,3 +139,49 @@ def test_sums_in_32_bits_are_as_good_as_the_streaming_kernels(monkeypatch, rows,
     ops.workspace().check_status()
     assert (y.double() - want).norm() <= 1.02 * off
     assert torch.equal(total, y + res) and torch.equal(y, ops.linear(x, w, out_f32=True))
+
+
+def _clamped(x, w, limit, slope):
+    """min(g, limit) sigmoid(slope g) (clamp(u, +-limit) + 1): clamping does not widen an error, z sigmoid(slope z) has a slope of at most 1.1 whatever `slope` is."""
+    (g, eg), (u, eu) = (_sum(x, h) for h in w.chunk(2))
+    g, u = g.clamp(max=limit), u.clamp(-limit, limit) + 1
+    s = g * torch.sigmoid(slope * g)
+    return s * u, (1.1 * eg + 2.0 ** -20 * s.abs()) * (u.abs() + eu) + (s.abs() + 1.1 * eg) * eu + 2.0 ** -22 * s.abs()
+
+
+# cut tiles and whole ones; limits that clamp many values and few
+@pytest.mark.parametrize("rows,features,K", [(300, 512, 2048), (2304, 2304, 256)])
+@pytest.mark.parametrize("limit,slope", [(0.5, 1.702), (7.0, 1.0)])
+def test_clamped_unit(monkeypatch, rows, features, K, limit, slope):
+    _pair_only(monkeypatch)
+    x, w = _inputs(rows, 2 * features, K)
+    _close(ops.swiglu_linear(x, w, glu=(limit, slope)), *_clamped(x, w, limit, slope))
+    cnt = torch.tensor([rows - 40, 0, 40], dtype=torch.int32, device=DEV)
+    off = torch.cat([cnt.new_zeros(1), cnt.cumsum(0).int()])
+    stack = torch.stack([w, w, -w])
+    y = ops.grouped_linear(x, stack, cnt, off, swiglu=True, glu=(limit, slope))
+    for i, at in ((0, slice(0, rows - 40)), (2, slice(rows - 40, rows))):
+        _close(y[at], *_clamped(x[at], stack[i], limit, slope))
+
+
+# an average that sends the product to the pairs, whatever the groups are: one with all rows, most of them empty, tiny ones beside a large one
+@pytest.mark.parametrize("counts", [[2048, 0, 0, 0, 0, 0, 0, 0], [0, 0, 1, 1990, 0, 57, 0, 0], [3, 700, 5, 0, 650, 1, 689, 0]])
+@pytest.mark.parametrize("unit", [False, True])
+def test_uneven_groups_by_their_average(monkeypatch, counts, unit):
+    monkeypatch.setattr(_lib.lib(), "skein_gemm_ws", None)          # the rule itself has to choose the pairs
+    features, K = (512, 512) if unit else (8192, 1536)
+    cnt = torch.tensor(counts, dtype=torch.int32, device=DEV)
+    off = torch.cat([cnt.new_zeros(1), cnt.cumsum(0).int()])
+    x, w = _inputs(sum(counts), features * (2 if unit else 1), K, lead=(8,))
+    y = ops.grouped_linear(x, w, cnt, off, swiglu=unit, rows_hint=2048)
+    for i, n in enumerate(counts):
+        at = slice(int(off[i]), int(off[i]) + n)
+        _close(y[at], *(_unit if unit else _sum)(x[at], w[i]))
+
+
+@pytest.mark.parametrize("rows,kernel", [(191, "skein_gemm_pair"), (192, "skein_gemm_ws"), (256, "skein_gemm_ws"), (257, "skein_gemm_pair"), (4200, "skein_gemm_ws")])
+def test_rule_at_its_edges(monkeypatch, rows, kernel):
+    """1024 features, K of 4096: the kernel that must not run is not there."""
+    monkeypatch.setattr(_lib.lib(), kernel, None)
+    x, w = _inputs(rows, 1024, 4096)
+    _close(ops.linear(x, w), *_sum(x, w))
