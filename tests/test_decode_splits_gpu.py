@@ -31,8 +31,8 @@ def _case(lens, Hq, Hkv, seed=0):
     return r(len(lens), (Hq + 2 * Hkv) * D), r(len(lens) * nb, 2, Hkv, PAGE, D), table, torch.tensor(lens, dtype=torch.int32, device="cuda")
 
 
-# a padding row, one token, around a tile, just below and above the lengths at which a second split begins, many splits
-LENS = [0, 1, 17, 383, 384, 385, 640, 1000, 2049]
+# a padding row, one token, around a tile, just below and above the lengths at which a second split begins (of 128 and of 256 tokens), many splits
+LENS = [0, 1, 17, 191, 192, 193, 383, 384, 385, 640, 1000, 2049]
 
 
 @pytest.mark.gpu
@@ -73,6 +73,7 @@ def test_rope_and_append_under_a_long_hint(lens):
     torch.cuda.synchronize()
     ops.workspace().check_status()
     assert torch.equal(*caches)
-    short = [i for i, n in enumerate(lens) if n < 384]
+    tokens = F.split_plan(len(lens), Hkv, 8192, ops.workspace().sm_count, Hq // Hkv)[1]
+    short = [i for i, n in enumerate(lens) if (n + tokens // 2) // tokens < 2]
     assert torch.equal(out[0][short], out[1][short])
     assert torch.allclose(out[0].float(), out[1].float(), atol=2.0 ** -6 * float(out[1].abs().max()))
