@@ -78,8 +78,9 @@ struct RouterOut {
 
 // Few tokens: grid = T, 512 threads: thread i owns 8 consecutive elements of the hidden vector per pass, so
 // every load of a pass is issued before the first is consumed. The last CTA to finish also lays out
-// the expert-sorted order (router_plan_body), which saves a launch on the decode path.
-__global__ void __launch_bounds__(512) router_topk_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ wg, int T, int H, int E,
+// the expert-sorted order (router_plan_body), which saves a launch on the decode path. Three CTAs per SM: with the layout's loads in flight the compiler
+// took registers for two, and 300 tokens, a third round of CTAs, 16.0 instead of 13.5 us (4 experts x 8192).
+__global__ void __launch_bounds__(512, 3) router_topk_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ wg, int T, int H, int E,
                                                           int topk, const RouterOut o) {
   __shared__ float part[16][RT_MAX_E];
   __shared__ float logit[RT_MAX_E];
