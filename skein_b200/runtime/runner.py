@@ -111,14 +111,14 @@ class _Bucket:
 
 
 class _Staging:
-    """Pinned buffers for the inputs of prefill chunks: a ring, each buffer guarded by the event behind its copy, made with the runner. (Taken
+    """Pinned buffers for the inputs of prefill chunks: a ring, each buffer guarded by the event behind its copy, the first made with the runner. (Taken
     from the host allocator for every chunk, the first chunk of each size class paid a page-locked allocation.) A buffer grows when a chunk is
     larger than any before it; the ring grows while all copies are still to come, up to RING, from where on the host waits."""
     WORDS, RING = 1 << 16, 8        # a 4096-token chunk of 64 sequences of up to 8192 tokens takes 45 thousand
 
     def __init__(self, device):
         self.device = device
-        self.ring = [self._make(self.WORDS), self._make(self.WORDS)] if device.type == "cuda" else []      # [buffer, event], oldest copy first
+        self.ring = [self._make(self.WORDS)] if device.type == "cuda" else []      # [buffer, event], oldest copy first
 
     @staticmethod
     def _make(words):

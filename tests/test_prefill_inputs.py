@@ -89,4 +89,4 @@ def test_one_buffer_grows_for_large_chunks():
         seqs = _chunk(i, 30000)
         _check(r._prefill_inputs(seqs, None)[0], seqs, 6)
         torch.cuda.synchronize()
-    assert sorted(s[0].numel() > _Staging.WORDS for s in r.staging.ring) == [False, True]
+    assert [s[0].numel() > _Staging.WORDS for s in r.staging.ring] == [True]
